@@ -43,6 +43,13 @@ struct SinCosConsts {
 	double w2 = -1. / 2, w4 = 1. / 24, w6 = -1. / 720, w8 = 1. / 40320;
 };
 
+// An addend of an integer-pipe square (nlc_intfp.cuh int_square_plus).
+struct IntAddend {
+	uint32_t lo, hi;   // significand, leading bit at bit 62 of 64
+	int32_t scale;     // biased exponent + 1023
+	uint32_t field;    // exponent field less the hidden bit
+};
+
 constexpr int kMaxSitesPerLane = 16;   // E: sites of a chain held in registers by one thread
 constexpr int kMaxLanesPerChain = 1024;
 
@@ -70,6 +77,7 @@ struct RealArgs {
 	double ck[7];          // kick coefficient dt * d[k]
 	double nck[7];         // -dt * d[k]
 	double mp2;            // DNKG: m + 2
+	IntAddend mp2_int;     // DNKG: m + 2 for the integer pipes
 	double alpha, beta;
 	double alpha2;         // Toda: 2 alpha
 	const double *mp2_site;  // dDNKG: m_x + 2 per site (device)

@@ -1,0 +1,117 @@
+// Double-precision operations on the integer pipes, correctly rounded (the bits of the FP64 unit).
+//
+// GB300 issues 2 FP64 lane-operations per SM and clock, one warp instruction per 64 clocks of a
+// scheduler, and the integrators saturate that pipe while the scheduler's other 60 issue slots pass
+// unused.  Logic, shifts, selects and comparisons issue at 64 lanes per SM and clock, IMAD at 64
+// beside them (a pipe of its own), 32-bit additions, minima and maxima at 128 (measured).  A double
+// addition written for these pipes takes 75 clocks of a scheduler against the FP64 pipe's 64, and
+// the two overlap: a DFMA beside it adds 6 clocks.  Sharing a sub-step's operations between the
+// pipes is therefore worth almost a second FP64 unit.
+//
+// The results are IEEE 754 round-to-nearest-even, bit for bit, so the CPU oracle replays the same
+// operations whichever pipe they ran on.  Operands for which the integer form does not hold (a sum
+// of zero or cancelled below the top 32 bits, magnitudes 2^32 apart, exponents near the ends of the
+// range, infinities and NaN) set a flag instead; the caller checks the flags of a batch of operations
+// with one vote and, where any lane has one set, redoes the batch on the FP64 pipe.
+#pragma once
+
+#include <cstdint>
+#include <cuda_runtime.h>
+
+#include "nlc_internal.h"
+
+namespace nlc {
+
+// What a batch of integer-pipe operations saw, as extremes (minima and maxima issue at twice the
+// rate of predicates): the batch is invalid when an exponent difference, an exponent or the high
+// word of a sum was out of the form's range.
+struct IntFlags {
+	uint32_t dmax = 0;    // largest exponent difference: up to 31
+	uint32_t exmax = 0;   // largest (biased exponent - 64), mod 2^32: up to 1976
+	int32_t rmin = 1;     // smallest high word of a sum, or alignment of a square: from 1
+	__device__ __forceinline__ bool bad() const { return (dmax > 31u) | (exmax > 1976u) | (rmin <= 0); }
+};
+
+__device__ __forceinline__ uint64_t mul_wide(uint32_t a, uint32_t b) {
+	uint64_t r;
+	asm("mul.wide.u32 %0, %1, %2;" : "=l"(r) : "r"(a), "r"(b));
+	return r;
+}
+__device__ __forceinline__ uint64_t mad_wide(uint32_t a, uint32_t b, uint64_t c) {
+	uint64_t r;
+	asm("mad.wide.u32 %0, %1, %2, %3;" : "=l"(r) : "r"(a), "r"(b), "l"(c));
+	return r;
+}
+__device__ __forceinline__ uint32_t lo32(uint64_t a) { return uint32_t(a); }
+__device__ __forceinline__ uint32_t hi32(uint64_t a) { return uint32_t(a >> 32); }
+
+// a - b.  Both significands are placed with the leading bit at bit 61 of 64 (carry at 62, sign at
+// 63), 9 bits below the last one kept; the smaller operand is shifted right, its lost bits ORed
+// into its lowest one, and added or (two's complement) subtracted; the sum's leading bit goes to
+// bit 62 and the 10 bits below the 53 kept are rounded off.  The hidden bit is added into the
+// exponent field, which also takes the carry of the rounding.
+__device__ __forceinline__ double int_sub(double a, double b, IntFlags &f) {
+	const uint32_t ah = __double2hiint(a), al = __double2loint(a), bh = __double2hiint(b) ^ 0x80000000u,
+	               bl = __double2loint(b);
+	const uint32_t aa = ah & 0x7fffffffu, ba = bh & 0x7fffffffu;
+	const bool swap = aa < ba;   // by the high words: equal ones cancel and are flagged where it matters
+	const uint32_t xh = swap ? bh : ah, xl = swap ? bl : al, yl = al + bl - xl;
+	const uint32_t xa = max(aa, ba), ya = min(aa, ba);
+	const uint32_t ex = xa >> 20, d = ex - (ya >> 20);
+	const uint32_t neg = uint32_t(int32_t(ah ^ bh) >> 31);   // all ones: magnitudes subtract
+	const uint32_t mx = (xa & 0xfffffu) | 0x100000u, my = (ya & 0xfffffu) | 0x100000u;
+	const uint32_t xhi = __funnelshift_l(xl, mx, 9), xlo = (xl << 9) - neg;   // the + 1 of the two's complement
+	const uint32_t yhi = __funnelshift_l(yl, my, 9), ylo = yl << 9;
+	const uint32_t lost = __funnelshift_r(0u, ylo, d);
+	const uint32_t slo = (__funnelshift_r(ylo, yhi, d) | min(lost, 1u)) ^ neg, shi = (yhi >> (d & 31u)) ^ neg;
+	uint32_t rl, rh;
+	asm("{add.cc.u32 %0, %2, %3; addc.u32 %1, %4, %5;}" : "=r"(rl), "=r"(rh) : "r"(xlo), "r"(slo), "r"(xhi), "r"(shi));
+	uint32_t lead;   // left shift that brings the leading bit of rh to bit 31
+	asm("bfind.shiftamt.u32 %0, %1;" : "=r"(lead) : "r"(rh));
+	const uint32_t s = lead - 1u;
+	const uint32_t nh = __funnelshift_l(rl, rh, s), nl = rl << (s & 31u);
+	const uint32_t half = ((nl >> 10) & 1u) + 0x1ffu;   // to nearest, ties to even
+	uint32_t ol, oh;
+	asm("{add.cc.u32 %0, %2, %3; addc.u32 %1, %4, 0;}" : "=r"(ol), "=r"(oh) : "r"(nl), "r"(half), "r"(nh));
+	f.dmax = max(f.dmax, d);
+	f.exmax = max(f.exmax, ex - 64u);
+	f.rmin = min(f.rmin, int32_t(rh));
+	return __hiloint2double(int(((oh >> 10) + (ex - s) * 0x100000u) | (xh & 0x80000000u)), int(__funnelshift_r(ol, oh, 10)));
+}
+
+// An addend K > 0 of int_square_plus: its significand with the leading bit at bit 62 of 64, its
+// exponent plus 1023, and the exponent field (less the hidden bit) that the result starts from.
+__device__ __forceinline__ IntAddend int_addend(double K) {
+	const uint32_t h = __double2hiint(K), l = __double2loint(K), m = (h & 0xfffffu) | 0x100000u;
+	return {l << 10, __funnelshift_l(l, m, 10), int32_t(h >> 20) + 1023, (h & 0x7ff00000u) - 0x100000u};
+}
+
+// c c + K for K of an ordinary positive exponent (the caller's check) and c c below K's next power of
+// two (flagged): the exact square of the 64-bit significand, shifted right to K's scale with the lost
+// bits ORed into the lowest one (bits of the square below 2^64 exist exactly when the significand's
+// low word is not zero), added to K's and rounded at K's exponent or the next.
+__device__ __forceinline__ double int_square_plus(double c, const IntAddend &K, IntFlags &f) {
+	const uint32_t ch = __double2hiint(c), cl = __double2loint(c);
+	const uint32_t mh = __funnelshift_l(cl, ch, 11) | 0x80000000u, ml = cl << 11;
+	const int32_t s = K.scale - 2 * int32_t((ch >> 20) & 0x7ffu);
+	// floor(m^2 / 2^64) = mh^2 + floor((mh ml + floor(ml^2 / 2^33)) / 2^31)
+	const uint64_t cross = mad_wide(mh, ml, uint64_t(hi32(mul_wide(ml, ml)) >> 1));
+	const uint64_t sq = mad_wide(mh, mh, cross >> 31);
+	uint64_t aligned, lost;
+	asm("shr.u64 %0, %1, %2;" : "=l"(aligned) : "l"(sq), "r"(s));        // shifts of 64 and more give 0
+	asm("shl.b64 %0, %1, %2;" : "=l"(lost) : "l"(sq), "r"(64 - s));
+	const uint32_t sticky = min(lo32(lost) | hi32(lost) | ml, 1u);
+	uint32_t rl, rh;
+	asm("{add.cc.u32 %0, %2, %3; addc.u32 %1, %4, %5;}"
+	    : "=r"(rl), "=r"(rh)
+	    : "r"(K.lo), "r"(lo32(aligned) | sticky), "r"(K.hi), "r"(hi32(aligned)));
+	const uint32_t carry = rh >> 31;                                     // the sum reached the next power of two
+	const uint32_t drop = 10u + carry, half = ((rl >> drop) & 1u) + (0x200u << carry) - 1u;
+	uint32_t ol, oh;
+	asm("{add.cc.u32 %0, %2, %3; addc.u32 %1, %4, 0;}" : "=r"(ol), "=r"(oh) : "r"(rl), "r"(half), "r"(rh));
+	const uint32_t top = oh >> drop;                                     // 0 where the rounding wrapped
+	f.rmin = min(f.rmin, min(s, int32_t(top)));
+	return __hiloint2double(int(top + K.field + carry * 0x100000u), int(__funnelshift_r(ol, oh, drop)));
+}
+
+}  // namespace nlc

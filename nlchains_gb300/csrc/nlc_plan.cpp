@@ -337,8 +337,25 @@ constexpr double kTuneMinSites = 65536;
 // Wall-clock budget of one tuning run; candidates after it are skipped, the best so far is kept.
 constexpr double kTuneBudgetMs = 150;
 
-// Time every launchable (G, threads) shape on a zero ensemble for a few steps (best of three
-// launches after a warm-up one); keep the fastest.  Small ensembles take the heuristic shape.
+// A small-amplitude ensemble for the tuner's launches: every site moving, no two alike (on zeros the
+// integrators' integer-pipe operations would all be redone in FP64, and the shapes rank differently).
+bool fill_tune_state(double *scratch, size_t doubles) {
+	std::vector<double> h(std::min<size_t>(doubles, size_t(1) << 17));
+	uint64_t s = 1;
+	for (double &v : h) {
+		s = s * 6364136223846793005ull + 1442695040888963407ull;
+		v = (double(s >> 11) * 0x1p-53 - 0.5) * 0.1;
+	}
+	if (cudaMemcpy(scratch, h.data(), h.size() * sizeof(double), cudaMemcpyHostToDevice) != cudaSuccess) return false;
+	for (size_t have = h.size(); have < doubles; have *= 2)
+		if (cudaMemcpy(scratch + have, scratch, std::min(have, doubles - have) * sizeof(double), cudaMemcpyDeviceToDevice) !=
+		    cudaSuccess)
+			return false;
+	return true;
+}
+
+// Time every launchable (G, threads) shape on a small-amplitude ensemble for a few steps (best of
+// three launches after a warm-up one); keep the fastest.  Small ensembles take the heuristic shape.
 RealShape autotune_shape(nlc_plan &P, int model, int variant) {
 	const TuneKey key{P.prop.name, model, variant, P.m.chain_length, copies_bucket(P.m.copies)};
 	{
@@ -366,7 +383,11 @@ RealShape autotune_shape(nlc_plan &P, int model, int variant) {
 		cudaGetLastError();
 		return fallback;
 	}
-	cudaMemset(scratch, 0, bytes);
+	if (!fill_tune_state(scratch, bytes / sizeof(double)) || cudaStreamSynchronize(cudaStreamLegacy) != cudaSuccess) {
+		cudaGetLastError();
+		cudaFree(scratch);
+		return fallback;
+	}
 	cudaStream_t st;
 	cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking);
 	cudaEvent_t e0, e1;
@@ -940,6 +961,14 @@ extern "C" int nlc_plan_create(const nlc_model *model, nlc_plan **out) {
 		a.cd0_merged = a.cd[0] * 2;
 		a.cd_final = kYoshidaC[7] * model->dt;
 		a.mp2 = model->m + 2;
+		{
+			// an addend of no ordinary positive exponent gets a scale that flags every square
+			uint64_t b;
+			std::memcpy(&b, &a.mp2, sizeof b);
+			const uint64_t e = b >> 52, sig = ((b & 0xfffffffffffffull) | 0x10000000000000ull) << 10;
+			const bool ok = e >= 64 && e <= 1983;
+			a.mp2_int = {uint32_t(sig), uint32_t(sig >> 32), ok ? int32_t(e) + 1023 : -8192, uint32_t(e - 1) << 20};
+		}
 		a.alpha = model->alpha, a.beta = model->beta;
 		a.alpha2 = 2 * model->alpha;
 		a.n = n, a.copies = model->copies;

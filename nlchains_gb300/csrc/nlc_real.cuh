@@ -18,19 +18,27 @@
 // * bond-based forces (FPUT, Toda) compute each bond once: a lane computes its own right bonds and
 //   receives the left bond of its first site from its left neighbour by shuffle, instead of
 //   recomputing it as the reference's RHS constructor does;
-// * every FP64 operation is an explicit round-to-nearest intrinsic in the order the CPU oracle
-//   replays (oracle/nlc_oracle.c, move_chain_device); adds and products are issued as FMAs with
-//   parameter-bank constants (bit-identical, faster issue on GB300, see nlc_device.cuh).
+// * every double operation is correctly rounded and in the order the CPU oracle replays
+//   (oracle/nlc_oracle.c, move_chain_device): an explicit round-to-nearest intrinsic, adds and
+//   products issued as FMAs with parameter-bank constants (bit-identical, faster issue on GB300, see
+//   nlc_device.cuh), or its integer-pipe form (nlc_intfp.cuh, the same bits).
 //
-// FP64 operations per site and sub-step (GB300 is FP64-pipe bound, see nlc_device.cuh):
-//   DNKG / dDNKG 6 (5 with beta == 1), FPUT 7 (6 with alpha == 0 and beta == 1),
-//   Toda 13 (12 with 2 alpha == 1) including the 8-operation table exp.
+// Operations per site and sub-step, and where they run (the FP64 pipe is the bound; the integer
+// pipes work beside it):
+//   DNKG / dDNKG 6 (5 with beta == 1): the subtraction and, with beta == 1, the square plus m + 2 on
+//     the integer pipes, 4 (3) left on the FP64 pipe.  DNKG N = 128, 65536 chains, 100 steps: 53.8
+//     ms with all five on the FP64 pipe, 39.8 with the subtraction moved, 32.1 with the square too
+//     (26.1 G site-steps/s; the FP64 pipe 87% busy at the three operations it keeps).
+//   FPUT 7 (6 with alpha == 0 and beta == 1), Toda 13 (12 with 2 alpha == 1) including the 8-operation
+//     table exp: the two subtractions on the integer pipes.  FPUT N = 459, 3001 chains, 50 steps: 7.05
+//     -> 5.54 ms; Toda N = 128, 16384 chains, 100 steps: 32.9 -> 28.5 ms.
 #pragma once
 
 #include <type_traits>
 
 #include "nlc_device.cuh"
 #include "nlc_internal.h"
+#include "nlc_intfp.cuh"
 
 namespace nlc {
 
@@ -107,8 +115,38 @@ __device__ __forceinline__ double bond_force(double d, const RealArgs &a, const 
 	}
 }
 
+// Integer-pipe operations are checked (and redone) this many sites at a time, so that a batch's
+// operands stay in registers until then.
+constexpr int kIntBatch = 8;
+
+// out[j] = a[j] - b[j], j < E.  INT: on the integer pipes; `last`: whether element E - 1 is used (a
+// short lane's last slot holds no site, and its flags are ignored).  Every lane of the warp calls it.
+template <int E, bool INT>
+__device__ __forceinline__ void sub_batch(double *out, const double *a, const double *b, bool last, const FpOnes &k) {
+	if constexpr (!INT) {
+#pragma unroll
+		for (int j = 0; j < E; j++) out[j] = fsub(a[j], b[j], k);
+	} else {
+#pragma unroll
+		for (int j0 = 0; j0 < E; j0 += kIntBatch) {
+			IntFlags f, fe;
+#pragma unroll
+			for (int j = j0; j < E && j < j0 + kIntBatch; j++) out[j] = int_sub(a[j], b[j], j == E - 1 ? fe : f);
+			if (__any_sync(0xffffffffu, f.bad() | (last & fe.bad()))) {
+#pragma unroll
+				for (int j = j0; j < E && j < j0 + kIntBatch; j++) out[j] = fsub(a[j], b[j], k);
+			}
+		}
+	}
+}
+
 template <int MODEL, int E, int VAR, bool WIN>
 __global__ void real_move_kernel_t(double2 *__restrict__ state, const RealArgs a) {
+	// Additions (and DNKG's squares) on the integer pipes beside the FP64 ones, from 4 sites per lane
+	// on.  Shapes of 2 or 3 sites per lane are those of ensembles too small to give a scheduler more
+	// than one or two warps: there the two pipes do not overlap (a warp issues in order), and an
+	// operation costs 75 clocks against 64.
+	constexpr bool INT = E >= 4;
 	__shared__ double xbuf[4 * 32];
 	__shared__ double s_tab[MODEL == NLC_TODA ? kExpTable : 1];
 	__shared__ unsigned long long s_unit;
@@ -135,6 +173,7 @@ __global__ void real_move_kernel_t(double2 *__restrict__ state, const RealArgs a
 	int full = 0, ne = 0, first = 0;
 	bool fl = false;
 	double mv[MODEL == NLC_DDNKG ? E : 1];
+	bool mv_bad = false;   // dDNKG: a lane's m + 2 whose exponent the integer squares do not take
 	constexpr bool windowed = WIN;
 	auto layout = [&]() {
 		// lanes [0, full) hold E sites, the others E - 1 (a window: G E sites, every lane E)
@@ -192,6 +231,7 @@ __global__ void real_move_kernel_t(double2 *__restrict__ state, const RealArgs a
 		}
 		const bool active = chain < copies;
 		if (!active) chain = copies - 1;   // redundant work keeps shuffles and barriers convergent
+		mv_bad = false;
 		double2 *cp = st + chain * (unsigned long long) n + (windowed ? 0 : first);
 
 		double x[E + 2], p[E];
@@ -209,8 +249,11 @@ __global__ void real_move_kernel_t(double2 *__restrict__ state, const RealArgs a
 			} else {
 				x[j + 1] = 0., p[j] = 0.;
 			}
+			if constexpr (INT && MODEL == NLC_DDNKG && VAR)
+				mv_bad |= uint32_t(__double2hiint(mv[j])) - 0x04000000u > 0x78000000u;
 		}
 
+		(void) mv_bad;
 		const double cd_lead = (seg & NLC_SEG_CONTINUE) ? a.cd0_merged : a.cd[0];
 		auto integrate = [&](auto shfl_tag) {
 		constexpr bool SHFL = decltype(shfl_tag)::value;
@@ -225,7 +268,7 @@ __global__ void real_move_kernel_t(double2 *__restrict__ state, const RealArgs a
 				for (int j = 0; j < E; j++) x[j + 1] = dfma(a.cd_final, p[j], x[j + 1]);
 			}
 			rpos++;
-#pragma unroll
+#pragma unroll (INT ? 1 : 7)
 			for (int k = 0; k < 7; k++) {
 				// the trailing drift of step i-1 (c[7]) merged with the leading drift of step i (c[0])
 				const double cd = k == 0 ? (i == 0 ? cd_lead : boundary ? a.cd[0] : a.cd0_merged) : a.cd[k];
@@ -237,28 +280,58 @@ __global__ void real_move_kernel_t(double2 *__restrict__ state, const RealArgs a
 					ring.template both<SHFL>(fl ? x[E] : x[E - 1], x[1], l, r);
 					x[0] = l, x[E + 1] = r;
 					if (!fl) x[E] = r;
-#pragma unroll
-					for (int j = 1; j <= E; j++) {
+					auto mp2 = [&](int j) {
+						if constexpr (MODEL == NLC_DDNKG) return mv[j - 1];
+						else return a.mp2;
+					};
+					auto force_fp64 = [&](int j) {
 						const double c = x[j];
 						const double bc = VAR ? c : fmul(a.beta, c, a.k1);
-						double mp2x;
-						if constexpr (MODEL == NLC_DDNKG) mp2x = mv[j - 1];
-						else mp2x = a.mp2;
-						const double t = dfma(bc, c, mp2x);
-						const double uu = dfma(c, t, -x[j - 1]);
-						const double v = fsub(uu, x[j + 1], a.k1);
-						p[j - 1] = dfma(a.nck[k], v, p[j - 1]);
+						return fsub(dfma(c, dfma(bc, c, mp2(j)), -x[j - 1]), x[j + 1], a.k1);
+					};
+					if constexpr (!INT) {
+#pragma unroll
+						for (int j = 1; j <= E; j++) p[j - 1] = dfma(a.nck[k], force_fp64(j), p[j - 1]);
+					} else {
+						// the square (beta = 1) and the subtraction on the integer pipes, a batch at a time
+#pragma unroll
+						for (int j0 = 1; j0 <= E; j0 += kIntBatch) {
+							IntFlags f, fe;
+							double v[kIntBatch];
+#pragma unroll
+							for (int j = j0; j <= E && j < j0 + kIntBatch; j++) {
+								IntFlags &fj = j == E ? fe : f;
+								const double c = x[j];
+								double t;
+								if constexpr (!VAR) {
+									t = dfma(fmul(a.beta, c, a.k1), c, mp2(j));
+								} else if constexpr (MODEL == NLC_DDNKG) {
+									t = int_square_plus(c, int_addend(mv[j - 1]), fj);
+								} else {
+									t = int_square_plus(c, a.mp2_int, fj);
+								}
+								v[j - j0] = int_sub(dfma(c, t, -x[j - 1]), x[j + 1], fj);
+							}
+							if (__any_sync(0xffffffffu, mv_bad | f.bad() | (fl & fe.bad()))) {
+#pragma unroll
+								for (int j = j0; j <= E && j < j0 + kIntBatch; j++) v[j - j0] = force_fp64(j);
+							}
+#pragma unroll
+							for (int j = j0; j <= E && j < j0 + kIntBatch; j++) p[j - 1] = dfma(a.nck[k], v[j - j0], p[j - 1]);
+						}
 					}
 				} else {
 					const double r = ring.template from_right<SHFL>(x[1]);
 					x[E + 1] = r;
 					if (!fl) x[E] = r;
-					double g[E + 1];
+					double g[E + 1], d[E];
+					sub_batch<E, INT>(d, x + 2, x + 1, fl, a.k1);
 #pragma unroll
-					for (int j = 1; j <= E; j++) g[j] = bond_force<MODEL, VAR>(fsub(x[j + 1], x[j], a.k1), a, s_tab);
+					for (int j = 1; j <= E; j++) g[j] = bond_force<MODEL, VAR>(d[j - 1], a, s_tab);
 					g[0] = ring.template from_left<SHFL>(fl ? g[E] : g[E - 1]);
+					sub_batch<E, INT>(d, g + 1, g, fl, a.k1);
 #pragma unroll
-					for (int j = 1; j <= E; j++) p[j - 1] = dfma(a.ck[k], fsub(g[j], g[j - 1], a.k1), p[j - 1]);
+					for (int j = 0; j < E; j++) p[j] = dfma(a.ck[k], d[j], p[j]);
 				}
 				if (!fl) p[E - 1] = 0.;   // the slot past a short lane's last site stays inert
 			}

@@ -1,0 +1,70 @@
+"""The integrators' integer-pipe operations (nlc_intfp.cuh) at operands where they can go wrong: bit for
+bit against the oracle, whose operations are the FP64 unit's.  Each ensemble mixes chains at rest, one
+excited site, exact nodes and equal neighbours (sums of zero, deep cancellation), dyadic values (ties),
+neighbours 2^40 apart, subnormal and very small values, and amplitudes beyond the squares' range."""
+import os
+
+import numpy as np
+import pytest
+
+import oracle as O
+from nlchains_gb300 import ic
+
+pytestmark = pytest.mark.gpu
+
+
+def edge_states(n, seed):
+    r = np.random.RandomState(seed)
+    s = np.arange(n)
+    rows = []
+
+    def add(phi, pi=None):
+        rows.append(np.stack((phi, np.zeros(n) if pi is None else pi), 1))
+
+    add(np.zeros(n))
+    add(np.where(s == n // 3, 0.3, 0.0))
+    add(-np.zeros(n), np.where(s == 0, -0.25, -0.0))
+    add(0.5 * np.sin(2 * np.pi * s / n), 0.1 * np.cos(2 * np.pi * s / n))
+    add(np.where(s % 4 == 0, 0.5, 0.0), np.where(s % 2 == 0, 0.25, -0.25))
+    add(r.randint(-8, 9, n) / 8.0, r.randint(-8, 9, n) / 16.0)
+    add(np.where(s % 2 == 0, 0.7, 0.7 * 2.0 ** -40) * r.uniform(0.5, 1, n))
+    add(0.3 + 1e-9 * r.standard_normal(n))
+    add(0.3 * (1 + 2.0 ** -52 * r.randint(0, 4, n)))
+    add(1e-310 * r.standard_normal(n), 1e-308 * r.standard_normal(n))
+    add(1e-200 * r.standard_normal(n), 1e-150 * r.standard_normal(n))
+    add(2.5 * r.standard_normal(n), r.standard_normal(n))
+    add(r.standard_normal(n) * 10.0 ** -r.randint(0, 30, n), r.standard_normal(n) * 10.0 ** -r.randint(0, 30, n))
+    add(0.4 * r.standard_normal(n), 0.4 * r.standard_normal(n))
+    return np.array(rows)
+
+
+# lanes x sites per lane: one warp with full lanes and short ones, up to and beyond a batch of 8, several
+# chains per warp, a block
+SHAPES = [(4, 1), (8, 1), (9, 1), (16, 1), (61, 8), (64, 8), (128, 16), (100, 8), (500, 32), (512, 64), (1000, 128)]
+MODELS = [("DNKG", dict(m=1.0, beta=1.0)), ("DNKG", dict(m=0.0, beta=1.0)), ("DNKG", dict(m=-2.5, beta=1.0)), ("DNKG", dict(m=-2.0, beta=1.0)),
+          ("DNKG", dict(m=0.3, beta=0.7)), ("dDNKG", dict(beta=1.0)), ("FPUT", dict(alpha=0.0, beta=1.0)),
+          ("FPUT", dict(alpha=0.25, beta=0.5)), ("Toda", dict(alpha=0.5)), ("Toda", dict(alpha=0.75))]
+
+
+@pytest.mark.parametrize("n,lanes", SHAPES)
+@pytest.mark.parametrize("model,params", MODELS, ids=lambda v: v if isinstance(v, str) else "-".join(map(str, v.values())))
+def test_bits_at_edge_operands(gpu, monkeypatch, model, params, n, lanes):
+    monkeypatch.setenv("NLC_FORCE_LANES", str(lanes))
+    masses = ic.masses_uniform(n, seed=n) if model == "dDNKG" else None
+    if masses is not None:
+        masses[n // 2] = -1.0   # an addend of 1 among those of 3 to 5
+    state = edge_states(n, n)
+    copies = len(state)
+    ctx = gpu.Context(0)
+    job = ctx.job(gpu.Model(model, n, copies, 0.05, masses=masses, **params), 4)
+    job.upload(state)
+    job.advance(8)
+    out = job.download()
+    job.close()
+    ctx.close()
+    exp = O.advance(O.Model(model, n, copies, 0.05, masses=masses, **params), state, 8, 4, order=O.ORDER_DEVICE)
+    exp = exp.reshape(copies, n, 2)
+    finite = np.isfinite(exp)
+    assert np.array_equal(finite, np.isfinite(out))
+    bad = (out.view(np.uint64) != exp.view(np.uint64)) & finite
+    assert not bad.any(), f"rows {np.unique(np.nonzero(bad)[0])}: {np.count_nonzero(bad)} values differ"
