@@ -5,7 +5,8 @@
 // the compiler's contraction choices; the CPU oracle replays the same sequence in C.  On GB300 the
 // FP64 pipe is the bottleneck of every integrator (600 G DFMA lane-ops/s for the whole GPU, ~1/58
 // of FP32), so these kernels are written to minimise FP64 instructions: integer and FP32 work,
-// shuffles and shared-memory traffic are comparatively free.
+// shuffles and shared-memory traffic are comparatively free, and some of the double operations
+// themselves run on the integer pipes (nlc_intfp.cuh).
 #pragma once
 
 #include <cstdint>
@@ -20,12 +21,37 @@ __device__ __forceinline__ double dadd(double a, double b) { return __dadd_rn(a,
 __device__ __forceinline__ double dsub(double a, double b) { return __dsub_rn(a, b); }
 __device__ __forceinline__ double dmul(double a, double b) { return __dmul_rn(a, b); }
 
-// On GB300 the FP64 pipe issues DFMA at 600 G lane-ops/s but DADD / DMUL at 506 G (measured with
-// runtime operands, independent of the values).  Adds, subtractions and multiplications on the hot
-// paths are therefore issued as FMAs with the exact same result: a + b = fma(a, 1, b),
-// a - b = fma(b, -1, a), a * b = fma(a, b, -0) (the -0 addend keeps the sign of a zero product).
-// The constants reach the kernels as parameters (FpOnes in nlc_internal.h), so the compiler cannot
-// fold them back into DADD / DMUL, and they are parameter-bank operands rather than registers.
+// On GB300 a DFMA whose three operands are vector registers occupies a scheduler's FP64 pipe for 64
+// clocks; one with a constant-bank or uniform-register operand for 76, and so do DADD and DMUL (all
+// measured, independent of the values).  Adds, subtractions and multiplications on the hot paths are
+// therefore issued as FMAs with the exact same result: a + b = fma(a, 1, b), a - b = fma(b, -1, a),
+// a * b = fma(a, b, -0) (the -0 addend keeps the sign of a zero product).  The constants come in as
+// kernel parameters (FpOnes in nlc_internal.h), so that the compiler cannot fold them back into
+// DADD / DMUL, and the kernels take vector-register copies of them and of their coefficients with
+// in_register.
+
+// zero for every thread, in a way that the compiler has to take for a value that differs between lanes
+__device__ __forceinline__ int lane_zero(const FpOnes &k) { return int(threadIdx.x >> k.lane_shift); }
+// the value in vector registers: what depends on a lane cannot stay in the constant bank or a uniform
+// register
+__device__ __forceinline__ double in_register(double v, int zero) {
+	return __hiloint2double(__double2hiint(v) ^ zero, __double2loint(v) ^ zero);
+}
+__device__ __forceinline__ FpOnes in_register(const FpOnes &k, int zero) {
+	FpOnes r = k;
+	r.one = in_register(k.one, zero), r.mone = in_register(k.mone, zero), r.mzero = in_register(k.mzero, zero);
+	return r;
+}
+// the constants of sincos_table's small-angle series (the others, of its table branch, stay where
+// they are: most angles are small)
+__device__ __forceinline__ SinCosConsts in_register(const SinCosConsts &c, int zero) {
+	SinCosConsts r = c;
+	r.q3 = in_register(c.q3, zero), r.q5 = in_register(c.q5, zero), r.q7 = in_register(c.q7, zero);
+	r.q9 = in_register(c.q9, zero), r.w2 = in_register(c.w2, zero), r.w4 = in_register(c.w4, zero);
+	r.w6 = in_register(c.w6, zero), r.w8 = in_register(c.w8, zero);
+	return r;
+}
+
 __device__ __forceinline__ double fadd(double a, double b, const FpOnes &k) { return __fma_rn(a, k.one, b); }
 __device__ __forceinline__ double fsub(double a, double b, const FpOnes &k) { return __fma_rn(b, k.mone, a); }
 __device__ __forceinline__ double fmul(double a, double b, const FpOnes &k) { return __fma_rn(a, b, k.mzero); }

@@ -1,4 +1,4 @@
-// DNLS split step with the linear sub-steps as a real-space stencil; chains resident in registers.
+// DNLS split step with the linear sub-steps as a real-space stencil; chains resident in shared memory.
 //
 // The linear sub-step of the reference, psi <- IFFT(FFT(psi) exp(-i tau omega_j) / n) with
 // tau = dt d_k and omega_j = 4 sin^2(pi j / n) = 2 - 2 cos(2 pi j / n) (DNLS.cpp:166-172,
@@ -12,35 +12,38 @@
 // so a linear sub-step is a (2R + 1)-point stencil with real coefficients and the factors i^x, which
 // only swap and negate real and imaginary parts.  The common phase exp(-2 i tau) is folded into the
 // angle of the nonlinear rotation that precedes the sub-step (both are diagonal in real space and
-// commute with |psi|).  FP64 operations per site and sub-step: the rotation 17 (norm 2, angle 1,
-// sincos 10 below 2^-4, product 4) and the stencil 4R + 2 (R symmetric sums psi_{s+x} + psi_{s-x},
-// R + 1 FMAs per component): 47 at R = 7, against 73 with the two shared-memory transforms at
-// n = 1024 (nlc_dnls.cu) and about twice that for a length with a large prime factor.  The centre
-// term is psi + (J_0 - 1) psi in one FMA, with J_0 - 1 held to full relative precision, so no
-// coefficient rounded near 1 scales the smooth modes the same way at every sub-step.
+// commute with |psi|).  Operations per site and sub-step: the rotation 17 (norm 2, angle 1, sincos 10
+// below 2^-4, product 4) and the stencil 4R + 2 (R symmetric sums psi_{s+x} + psi_{s-x}, R + 1 FMAs per
+// component): 47 at R = 7, against 73 with the two shared-memory transforms at n = 1024 (nlc_dnls.cu)
+// and about twice that for a length with a large prime factor.  The centre term is psi + (J_0 - 1) psi
+// in one FMA, with J_0 - 1 held to full relative precision, so no coefficient rounded near 1 scales the
+// smooth modes the same way at every sub-step.
 //
-// Layout: a chain of n sites on G lanes (any G up to 256), each lane holding E or E - 1 consecutive
-// sites (E in {8, 12, 16}, the first n - G (E - 1) lanes holding E) plus R halo sites on each side.
-// G <= 32: floor(32 / G) chains per warp, halos by shuffles from explicit lanes, no barrier;
-// G > 32: one chain per block, halos by shuffles inside warps and through shared memory across
-// them, one barrier per sub-step.  The grid is persistent (self-resetting work counter) as for the
-// real models.
+// The FP64 pipe is the bound, so the 2R sums and 5 of the rotation's products run on the integer pipes
+// (nlc_intfp.cuh, the same bits), 28 operations at R = 7 stay on the FP64 pipe, and every operand of
+// theirs is a vector register.  n = 1024, 8192 chains, 10 steps: 51.8 ms with all 47 on the FP64 pipe,
+// 32.9 with the sums moved (that pipe 99% busy), 28.4 with the products too (2.95 G site-steps/s).
 //
-// Chains longer than one block holds (WIN): windows of G E sites of the periodic chain (every lane
-// full), advanced a few steps per launch as if the window were a ring.  A sub-step moves
-// information R sites, so after s steps only the 7 R s sites at each end of the window have seen
-// the false wrap-around; the interior between them is exact and is written to the second buffer,
-// and the windows' interiors tile the chain.
+// Layout: a chain in shared memory, real and imaginary rows, twice (a sub-step reads one buffer and
+// writes the other), the R elements at each end of a row repeating the ring's other end.  G lanes (up
+// to 256) take its sites row by row (site r G + lane), E or E - 1 of them each, one component at a
+// time: 15 loads, 7 sums and 8 FMAs at R = 7 keep the kernel at 80 registers (unrolled over a lane's
+// sites in registers, the integer sums of several sites interleave and spill).  G <= 32: floor(32 / G)
+// chains per warp, no barrier; G > 32: one chain per block, one barrier per sub-step.  The grid is
+// persistent (self-resetting work counter) as for the real models.
+//
+// Chains longer than one block holds (WIN): windows of G E sites of the periodic chain, advanced a few
+// steps per launch as if the window were a ring.  A sub-step moves information R sites, so after s
+// steps only the 7 R s sites at each end of the window have seen the false wrap-around; the interior
+// between them is exact and is written to the second buffer, and the windows' interiors tile the
+// chain.
 #include "nlc_device.cuh"
 #include "nlc_internal.h"
+#include "nlc_intfp.cuh"
 
 namespace nlc {
 
 namespace {
-
-__device__ __forceinline__ double2 shfl2(double2 v, int src) {
-	return make_double2(__shfl_sync(0xffffffffu, v.x, src), __shfl_sync(0xffffffffu, v.y, src));
-}
 
 // psi exp(i (neg_coef |psi|^2 + neg_phase)): the nonlinear rotation with the propagator's phase
 __device__ __forceinline__ double2 rotate_phase(double2 v, double neg_coef, double neg_phase,
@@ -52,42 +55,109 @@ __device__ __forceinline__ double2 rotate_phase(double2 v, double neg_coef, doub
 	return make_double2(dfma(v.x, c, -fmul(v.y, s, k)), dfma(v.x, s, fmul(v.y, c, k)));
 }
 
+// The same with the products of two varying factors on the integer pipes (5 of the 17 operations of an
+// angle below 2^-4); redone by rotate_phase where a lane's operands ask for it.  Every lane of the
+// warp calls it.
+__device__ __forceinline__ double2 rotate_phase_mixed(double2 v, double neg_coef, double neg_phase,
+                                                      const double2 *__restrict__ sctab, const SinCosConsts &C,
+                                                      const FpOnes &k) {
+	IntFlags f;
+	const double th = dfma(neg_coef, dfma(v.x, v.x, int_mul(v.y, v.y, f)), neg_phase);
+	double s, c;
+	if (__all_sync(0xffffffffu, (__double2hiint(th) & 0x7fffffff) < 0x3fb00000)) {   // sincos_table's series
+		const double t2 = int_mul(th, th, f);
+		const double ps = dfma(t2, dfma(t2, dfma(t2, C.q9, C.q7), C.q5), C.q3);
+		s = dfma(int_mul(th, t2, f), ps, th);
+		c = dfma(t2, dfma(t2, dfma(t2, dfma(t2, C.w8, C.w6), C.w4), C.w2), k.one);
+	} else {
+		sincos_table(th, sctab, C, k, &s, &c);
+	}
+	const double2 r = make_double2(dfma(v.x, c, -int_mul(v.y, s, f)), dfma(v.x, s, int_mul(v.y, c, f)));
+	return __any_sync(0xffffffffu, f.bad()) ? rotate_phase(v, neg_coef, neg_phase, sctab, C, k) : r;
+}
+
 }  // namespace
+
+// One component (the real or the imaginary part) of the (2R + 1)-point stencil at one site:
+// psi + (J_0 - 1) psi + sum_x J_x i^x (psi_{s+x} + psi_{s-x}).  `own` and `other` point at the site's
+// component and its counterpart; the factor i of odd x takes the sums from `other`, and the taps carry
+// the signs.  `add` forms the sums.
+template <int R, class Add>
+__device__ __forceinline__ double stencil_component(const double *own, const double *other, const double *tp, Add add) {
+	double y = dfma(tp[0], own[0], own[0]);
+#pragma unroll
+	for (int x = 1; x <= R; x++) {
+		const double *w = x & 1 ? other : own;
+		y = dfma(tp[x], add(w[x], w[-x]), y);
+	}
+	return y;
+}
+
+// double2s of the constants ahead of the buffers: the taps, the rotations, the sine and cosine series
+template <int R>
+constexpr int kStencilConsts = 7 * (R + 1) + 9 + 4;
 
 // TEAM: G <= 32, 128-thread blocks; otherwise one chain (WIN: one window) per block of ceil(G / 32)
 // warps
-template <int E, int R, bool TEAM, bool WIN>
-__global__ void __launch_bounds__(TEAM ? 128 : 256) dnls_stencil_kernel(double2 *__restrict__ psi, const DnlsStencilArgs a) {
-	static_assert(E - 1 >= R, "a lane's halo comes from one neighbour: E - 1 >= R sites");
+template <int R, bool TEAM, bool WIN>
+__global__ void __launch_bounds__(TEAM ? 128 : WIN ? 384 : 256, WIN ? 2 : (TEAM ? 2 : 1) * (R <= 7 ? 3 : 2)) dnls_stencil_kernel(double2 *__restrict__ psi, const DnlsStencilArgs a) {
 	static_assert(!(WIN && TEAM), "windows are block-wide");
-	// G > 32: the halos crossing warps, [2 parities][2 directions][warps][R]
-	extern __shared__ double2 xb[];
+	// per chain (window): two buffers of two rows of R + len + R doubles, the R at each end the ring's other end
+	extern __shared__ double2 sm[];
 	__shared__ unsigned long long s_unit;
-	const int G = a.lanes, n = int(a.n), tid = threadIdx.x;
+	const int G = a.lanes, n = int(a.n), len = WIN ? int(a.win_len) : n, tid = threadIdx.x;
 	const int wl = tid & 31, warp = tid >> 5;
 	const int per_warp = TEAM ? 32 / G : 1;
 	const int cw = TEAM ? wl / G : 0;                    // chain of this lane within its warp
 	const bool spare = TEAM && cw >= per_warp;           // lanes past the warp's last whole chain
 	const int lane = TEAM ? (spare ? 0 : wl - cw * G) : tid;
 	const int gpb = TEAM ? per_warp * int(blockDim.x >> 5) : 1;   // chains per block
-	const int gib = TEAM ? warp * per_warp + cw : 0;
-	const int W = TEAM ? 1 : (G + 31) >> 5;
-	const bool idle = spare || lane >= G;                // lanes that hold no sites (never stored)
-	// neighbour lanes (within the warp; G > 32: the warp-edge and wrap-around pairs go through
-	// shared memory)
-	const int src_left = TEAM ? (spare ? wl : cw * G + (lane + G - 1) % G) : ((wl + 31) & 31);
-	const int src_right = TEAM ? (spare ? wl : cw * G + (lane + 1) % G) : ((wl + 1) & 31);
-	const bool left_smem = !TEAM && !idle && (wl == 0 || lane == 0);
-	const bool right_smem = !TEAM && !idle && (wl == 31 || lane == G - 1);
-	const int left_warp = lane == 0 ? ((G - 1) >> 5) : warp - 1;   // warp of lane - 1 (mod G)
-	const int right_warp = lane == G - 1 ? 0 : warp + 1;            // warp of lane + 1 (mod G)
+	const int gib = TEAM ? warp * per_warp + (spare ? 0 : cw) : 0;   // (a spare lane reads its warp's first chain)
+	const bool idle = spare || lane >= G;                // lanes that hold no sites (they read, never write)
+	const int rows = (len + G - 1) / G;
+	const int pitch = len + 2 * R;
+	double *const buf0 = reinterpret_cast<double *>(sm + kStencilConsts<R>) + size_t(gib) * 4 * pitch + R;
+	// The kernel's constants, in the shared memory of the buffers: DFMA operands loaded from there are
+	// vector registers (nlc_device.cuh), and at each use anew, which keeps the kernel at 80 registers.
+	// tap_sm: c0m1 and the R taps of each sub-step and component (the real part's odd taps negated);
+	// rot_sm: angle coefficient and phase of each sub-step's rotation, [7] the launch's first, [8] its
+	// closing one
+	double *const tap_sm = reinterpret_cast<double *>(sm);
+	double2 *const rot_sm = sm + 7 * (R + 1);
+	double *const ser_sm = reinterpret_cast<double *>(rot_sm + 9);
+	for (int i = tid; i < 14 * (R + 1); i += blockDim.x) {
+		const int row = i / (R + 1), x = i - row * (R + 1), k = row >> 1;
+		tap_sm[i] = !x ? a.c0m1[k] : (x & 1) && !(row & 1) ? -a.taps[k][x - 1] : a.taps[k][x - 1];
+	}
+	if (tid < 9) {
+		const bool merged = tid == 0 || (tid == 7 && (a.seg & NLC_SEG_CONTINUE));
+		rot_sm[tid] = make_double2(-(tid == 8 ? a.nl_final : merged ? a.nl[7] : a.nl[tid % 7]), tid == 8 ? 0. : a.phase[tid % 7]);
+	}
+	if (tid == 0) {
+		ser_sm[0] = a.sc.q3, ser_sm[1] = a.sc.q5, ser_sm[2] = a.sc.q7, ser_sm[3] = a.sc.q9;
+		ser_sm[4] = a.sc.w2, ser_sm[5] = a.sc.w4, ser_sm[6] = a.sc.w6, ser_sm[7] = a.sc.w8;
+	}
+	const int zero = lane_zero(a.k1);
+	const FpOnes k1 = in_register(a.k1, zero);
+	auto rotate = [&](double2 v, int i) {
+		SinCosConsts sc = a.sc;
+		sc.q3 = ser_sm[0], sc.q5 = ser_sm[1], sc.q7 = ser_sm[2], sc.q9 = ser_sm[3];
+		sc.w2 = ser_sm[4], sc.w4 = ser_sm[5], sc.w6 = ser_sm[6], sc.w8 = ser_sm[7];
+		const double2 c = rot_sm[i];
+		return rotate_phase_mixed(v, c.x, c.y, a.sctab, sc, k1);
+	};
 
-	const int full = WIN ? G : n - G * (E - 1);
-	const bool fl = lane < full;
-	const int ne = fl ? E : E - 1;
-	const int first = fl ? lane * E : full * E + (lane - full) * (E - 1);
-	const FpOnes &k1 = a.k1;
-	int parity = 0;
+	auto sync = [] {
+		if (TEAM) __syncwarp();
+		else __syncthreads();
+	};
+	// element s of a buffer (its real parts, then its imaginary ones), and its copy beyond the ring's
+	// other end
+	auto put = [&](double *buf, int s, double2 v) {
+		buf[s] = v.x, buf[pitch + s] = v.y;
+		if (s < R) buf[len + s] = v.x, buf[pitch + len + s] = v.y;
+		if (s >= len - R) buf[s - len] = v.x, buf[pitch + s - len] = v.y;
+	};
 
 	const unsigned long long units =
 	    WIN ? (unsigned long long) a.copies * a.win_count : (a.copies + gpb - 1) / gpb;
@@ -99,121 +169,67 @@ __global__ void __launch_bounds__(TEAM ? 128 : 256) dnls_stencil_kernel(double2 
 		if (u >= units) break;
 		unsigned long long chain = WIN ? u / a.win_count : u * gpb + gib;
 		const uint32_t win = WIN ? uint32_t(u - chain * a.win_count) : 0;
-		// WIN: the chain site of this lane's first site (the window starts win_halo sites before its
-		// interior)
-		const uint32_t wsite = WIN ? uint32_t((win * (unsigned long long) a.win_inner + n - a.win_halo + first) % n) : 0;
+		// WIN: the chain site of the window's first site, win_halo sites before its interior
+		const uint32_t wsite = WIN ? uint32_t((win * (unsigned long long) a.win_inner + n - a.win_halo) % n) : 0;
 		const bool active = chain < a.copies && !idle;
-		if (chain >= a.copies) chain = a.copies - 1;   // redundant work keeps shuffles and barriers convergent
-		double2 *g = psi + chain * (unsigned long long) n + (idle || WIN ? 0 : first);
+		if (chain >= a.copies) chain = a.copies - 1;   // redundant work keeps votes and barriers convergent
+		double2 *g = psi + chain * (unsigned long long) n;
 
-		// w: [0, R) left halo, [R, R + E) this lane's sites, [R + E, R + E + R) right halo; a short
-		// lane's slot R + E - 1 is inert (zero) between sub-steps
-		double2 w[E + 2 * R];
-#pragma unroll
-		for (int j = 0; j < E; j++) {
-			uint32_t sj = j;
+		double *in = buf0, *out = buf0 + 2 * pitch;
+		for (int r = 0; r < rows; r++) {
+			const int s = r * G + lane;
+			const bool mine = !idle && s < len;
+			uint32_t gs = mine ? s : 0;
 			if (WIN) {
-				sj = wsite + j;
-				if (sj >= uint32_t(n)) sj -= n;
+				gs += wsite;
+				if (gs >= uint32_t(n)) gs -= n;
 			}
-			w[R + j] = (!idle && j < ne) ? g[sj] : make_double2(0., 0.);
+			const double2 v = rotate(g[gs], 7);
+			if (mine) put(in, s, v);
 		}
-
-		for (uint32_t i = 0; i < a.steps; i++) {
+		sync();
+		const unsigned long long subs = 7ull * a.steps;
+		int k = 0;
+		for (unsigned long long i = 0; i < subs; i++) {
+			const double *const tp = tap_sm + 2 * k * (R + 1);
+			const bool last = i + 1 == subs;
+			k = k == 6 ? 0 : k + 1;
+			const int next = last ? 8 : k;   // the next rotation: the next sub-step's, or the launch's closing one
 #pragma unroll 1
-			for (int k = 0; k < 7; k++) {
-				const double nc = -((k == 0 && (i != 0 || (a.seg & NLC_SEG_CONTINUE))) ? a.nl[7] : a.nl[k]);
-				const double ph = a.phase[k];
-#pragma unroll
-				for (int j = 0; j < E; j++) w[R + j] = rotate_phase(w[R + j], nc, ph, a.sctab, a.sc, k1);
-
-				// halos: the left one is lane - 1's last R sites, the right one lane + 1's first R
-				double2 rl[R], rr[R];
-#pragma unroll
-				for (int x = 0; x < R; x++) {
-					const double2 last = fl ? w[E + x] : w[E - 1 + x];   // site ne - R + x
-					rl[x] = shfl2(last, src_left);
-					rr[x] = shfl2(w[R + x], src_right);
+			for (int r = 0; r < rows; r++) {
+				const int s = r * G + lane;
+				const bool mine = !idle && s < len;
+				const double *w = in + (mine ? s : 0);
+				double2 y = make_double2(0., 0.);
+#pragma unroll 1
+				for (int c = 0; c < 2; c++) {
+					const double *own = w + c * pitch, *other = w + (1 - c) * pitch, *t = tp + c * (R + 1);
+					// the sums on the integer pipes; redone on the FP64 pipe where a lane's operands ask for it
+					IntFlags f;
+					double v = stencil_component<R>(own, other, t, [&](double u, double v) { return int_add(u, v, f); });
+					if (__any_sync(0xffffffffu, f.bad()))
+						v = stencil_component<R>(own, other, t, [&](double u, double v) { return fadd(u, v, k1); });
+					if (c) y.y = v;
+					else y.x = v;
 				}
-				if (!TEAM) {
-					double2 *buf = xb + parity * 2 * W * R;
-					if (right_smem) {
-#pragma unroll
-						for (int x = 0; x < R; x++) buf[warp * R + x] = fl ? w[E + x] : w[E - 1 + x];
+				if (!last || !(a.seg & NLC_SEG_OPEN)) y = rotate(y, next);
+				if (!last) {
+					if (mine) put(out, s, y);
+				} else if (active && mine) {
+					if (WIN) {
+						// the interior's sites, to win_out
+						const uint32_t base = win * a.win_inner;   // chain site of the interior's first site
+						const uint32_t inner = min(a.win_inner, uint32_t(n) - base), at = uint32_t(s) - a.win_halo;
+						if (uint32_t(s) >= a.win_halo && at < inner)
+							a.win_out[chain * (unsigned long long) n + base + at] = y;
+					} else {
+						g[s] = y;
 					}
-					if (left_smem) {
-#pragma unroll
-						for (int x = 0; x < R; x++) buf[(W + warp) * R + x] = w[R + x];
-					}
-					__syncthreads();
-					if (left_smem) {
-#pragma unroll
-						for (int x = 0; x < R; x++) rl[x] = buf[left_warp * R + x];
-					}
-					if (right_smem) {
-#pragma unroll
-						for (int x = 0; x < R; x++) rr[x] = buf[(W + right_warp) * R + x];
-					}
-					parity ^= 1;
 				}
-#pragma unroll
-				for (int x = 0; x < R; x++) w[x] = rl[x];
-				// the right halo follows the lane's last site: slot R + E on a full lane, R + E - 1 on a
-				// short one (its inert slot)
-				w[R + E - 1] = fl ? w[R + E - 1] : rr[0];
-#pragma unroll
-				for (int x = 0; x < R - 1; x++) w[R + E + x] = fl ? rr[x] : rr[x + 1];
-				w[R + E + R - 1] = rr[R - 1];
-
-				// the stencil: psi + (J_0 - 1) psi + sum_x J_x i^x (psi_{s+x} + psi_{s-x}), the sign of
-				// i^x folded into taps (x = 2, 3 mod 4 negative), the factor i of odd x as a swap
-				const double c0 = a.c0m1[k];
-				double tp[R];
-#pragma unroll
-				for (int x = 0; x < R; x++) tp[x] = a.taps[k][x];
-				double2 y[E];
-#pragma unroll
-				for (int j = 0; j < E; j++) {
-					const double2 c = w[R + j];
-					double yr = dfma(c0, c.x, c.x), yi = dfma(c0, c.y, c.y);
-#pragma unroll
-					for (int x = 1; x <= R; x++) {
-						const double sr = fadd(w[R + j + x].x, w[R + j - x].x, k1);
-						const double si = fadd(w[R + j + x].y, w[R + j - x].y, k1);
-						if (x & 1) {
-							yr = dfma(-tp[x - 1], si, yr);
-							yi = dfma(tp[x - 1], sr, yi);
-						} else {
-							yr = dfma(tp[x - 1], sr, yr);
-							yi = dfma(tp[x - 1], si, yi);
-						}
-					}
-					y[j] = make_double2(yr, yi);
-				}
-#pragma unroll
-				for (int j = 0; j < E; j++) w[R + j] = y[j];
-				if (!fl) w[R + E - 1] = make_double2(0., 0.);
 			}
-		}
-		if (active) {
-			const bool open = a.seg & NLC_SEG_OPEN;
-			double2 *dst = g;
-			// WIN: the interior's window positions [lo, hi) relative to this lane's first site, and the
-			// chain site of this lane's first site, written to win_out
-			int lo = 0, hi = E;
-			long long site0 = 0;
-			if (WIN) {
-				const uint32_t base = win * a.win_inner;   // chain site of the interior's first site
-				const uint32_t inner = min(a.win_inner, uint32_t(n) - base);
-				dst = a.win_out + chain * (unsigned long long) n;
-				lo = int(a.win_halo) - first;
-				hi = int(a.win_halo + inner) - first;
-				site0 = (long long) base - a.win_halo + first;
-			}
-#pragma unroll
-			for (int j = 0; j < E; j++)
-				if (j < ne && j >= lo && j < hi)
-					dst[site0 + j] = open ? w[R + j] : rotate_phase(w[R + j], -a.nl_final, 0., a.sctab, a.sc, k1);
+			sync();
+			double *const swap = in;
+			in = out, out = swap;
 		}
 	}
 
@@ -233,54 +249,44 @@ namespace {
 
 using StencilKernel = void (*)(double2 *, const DnlsStencilArgs);
 
-StencilKernel stencil_kernel(int sites, int radius, bool team, bool win) {
-	if (win) {   // windows: 16 sites per lane
-		if (sites != 16 || team) return nullptr;
-		return radius == 7 ? dnls_stencil_kernel<16, 7, false, true>
-		                   : radius == 11 ? dnls_stencil_kernel<16, 11, false, true> : nullptr;
-	}
-	if (radius == 7) {
-		switch (sites) {
-			case 8: return team ? dnls_stencil_kernel<8, 7, true, false> : dnls_stencil_kernel<8, 7, false, false>;
-			case 12: return team ? dnls_stencil_kernel<12, 7, true, false> : dnls_stencil_kernel<12, 7, false, false>;
-			case 16: return team ? dnls_stencil_kernel<16, 7, true, false> : dnls_stencil_kernel<16, 7, false, false>;
-		}
-	} else if (radius == 11) {
-		switch (sites) {
-			case 12: return team ? dnls_stencil_kernel<12, 11, true, false> : dnls_stencil_kernel<12, 11, false, false>;
-			case 16: return team ? dnls_stencil_kernel<16, 11, true, false> : dnls_stencil_kernel<16, 11, false, false>;
-		}
-	}
-	return nullptr;
+template <int R>
+StencilKernel stencil_kernel_of(bool team, bool win) {
+	return win ? dnls_stencil_kernel<R, false, true> : team ? dnls_stencil_kernel<R, true, false>
+	                                                        : dnls_stencil_kernel<R, false, false>;
+}
+
+StencilKernel stencil_kernel(int radius, bool team, bool win) {
+	if (win && team) return nullptr;
+	return radius == 7 ? stencil_kernel_of<7>(team, win) : radius == 11 ? stencil_kernel_of<11>(team, win) : nullptr;
 }
 
 }  // namespace
 
-const void *dnls_stencil_kernel_ptr(int sites, int radius, bool team, bool windowed) {
-	return (const void *) stencil_kernel(sites, radius, team, windowed);
+const void *dnls_stencil_kernel_ptr(int radius, bool team, bool windowed) {
+	return (const void *) stencil_kernel(radius, team, windowed);
 }
 
-size_t dnls_stencil_smem(int lanes, int radius) {
-	return lanes > 32 ? size_t(4) * ((lanes + 31) / 32) * radius * sizeof(double2) : 0;
+size_t dnls_stencil_smem(uint32_t len, int lanes, int radius) {
+	const size_t chains = lanes > 32 ? 1 : size_t(4) * (32 / lanes);
+	const size_t consts = radius == 7 ? kStencilConsts<7> : kStencilConsts<11>;
+	return (consts + chains * 2 * (len + 2 * size_t(radius))) * sizeof(double2);
 }
 
-cudaError_t launch_dnls_stencil(const DnlsStencilArgs &a, double2 *psi, int sites, int radius, int blocks,
-                                cudaStream_t stream) {
+cudaError_t launch_dnls_stencil(const DnlsStencilArgs &a, double2 *psi, int radius, int blocks, cudaStream_t stream) {
 	const bool team = a.lanes <= 32;
-	const StencilKernel k = stencil_kernel(sites, radius, team, a.win_len != 0);
-	if (!k || a.lanes < 1 || a.lanes > 256 || !a.copies || blocks < 1) return cudaErrorInvalidConfiguration;
+	const StencilKernel k = stencil_kernel(radius, team, a.win_len != 0);
+	if (!k || a.lanes < 1 || a.lanes > (a.win_len ? 384 : 256) || !a.copies || !a.steps || blocks < 1) return cudaErrorInvalidConfiguration;
 	if (a.win_len) {
-		// a window fills every lane, lies inside the chain, and keeps a non-empty interior
-		if (a.win_len != uint32_t(a.lanes) * uint32_t(sites) || a.n <= a.win_len || !a.win_inner ||
-		    2ull * a.win_halo + a.win_inner > a.win_len || !a.win_out ||
+		// a window lies inside the chain and keeps a non-empty interior
+		if (a.lanes <= 32 || a.n <= a.win_len || !a.win_inner || 2ull * a.win_halo + a.win_inner > a.win_len || !a.win_out ||
 		    a.win_count != (a.n + a.win_inner - 1) / a.win_inner)
 			return cudaErrorInvalidConfiguration;
-	} else if (uint64_t(a.lanes) * (sites - 1) >= a.n || uint64_t(a.lanes) * sites < a.n || a.n < uint32_t(2 * radius + 2)) {
-		return cudaErrorInvalidConfiguration;   // every lane holds sites or sites - 1 >= radius sites
+	} else if (a.n < uint32_t(2 * radius + 2)) {
+		return cudaErrorInvalidConfiguration;
 	}
 	count_launch();
 	const int threads = team ? 128 : (a.lanes + 31) / 32 * 32;
-	k<<<blocks, threads, dnls_stencil_smem(a.lanes, radius), stream>>>(psi, a);
+	k<<<blocks, threads, dnls_stencil_smem(a.win_len ? a.win_len : a.n, a.lanes, radius), stream>>>(psi, a);
 	return cudaGetLastError();
 }
 

@@ -10,11 +10,12 @@
 
 namespace nlc {
 
-// FP64 constants that reach the kernels as parameters rather than literals: on GB300 an FMA whose
-// constant operands come from the parameter bank issues faster than one with literal operands or
-// than DADD / DMUL, so the hot paths issue adds and products as FMAs with these (see nlc_device.cuh).
+// FP64 constants that reach the kernels as parameters rather than literals, so that the compiler does
+// not fold the FMAs that adds and products are issued as back into DADD and DMUL (see
+// nlc_device.cuh); lane_shift makes the zero of in_register there.
 struct FpOnes {
 	double one = 1., mone = -1., mzero = -0.;
+	uint32_t lane_shift = 31;
 };
 // Constants of the table-driven exp (nlc_device.cuh exp_scaled).
 constexpr int kExpTable = 2048;   // entries of the table exp: 2^(j/2048), |r| <= ln 2 / 4096
@@ -242,9 +243,8 @@ struct DnlsArgs {
 };
 cudaError_t launch_dnls_move(const DnlsArgs &a, double2 *psi, int blocks, int threads, size_t smem,
                              int team_block, cudaStream_t stream);
-// DNLS with the linear sub-steps as a real-space stencil (nlc_dnls_stencil.cu): chains of n sites on
-// `lanes` lanes of E or E - 1 sites in registers, stencil radius R (instantiated: E in {8, 12, 16}
-// with R = 7, E in {12, 16} with R = 11)
+// DNLS with the linear sub-steps as a real-space stencil (nlc_dnls_stencil.cu) of radius R (instantiated: 7
+// and 11), the sites of a chain (or window) taken row by row by `lanes` threads
 constexpr int kMaxStencilRadius = 11;
 struct DnlsStencilArgs {
 	uint32_t n, copies, steps, seg;
@@ -257,16 +257,15 @@ struct DnlsStencilArgs {
 	const double2 *sctab;
 	SinCosConsts sc;
 	FpOnes k1;
-	// windowed launches (chains beyond one block, win_len != 0): windows of win_len = lanes x E
-	// sites, every lane full, win_halo sites at each end recomputed and discarded, the interiors
-	// written to win_out
+	// windowed launches (chains beyond one block, win_len != 0): windows of win_len sites, win_halo
+	// sites at each end recomputed and discarded, the interiors written to win_out
 	uint32_t win_len, win_halo, win_inner, win_count;
 	double2 *win_out;
 };
-cudaError_t launch_dnls_stencil(const DnlsStencilArgs &a, double2 *psi, int sites, int radius, int blocks,
-                                cudaStream_t stream);
-const void *dnls_stencil_kernel_ptr(int sites, int radius, bool team, bool windowed = false);
-size_t dnls_stencil_smem(int lanes, int radius);
+cudaError_t launch_dnls_stencil(const DnlsStencilArgs &a, double2 *psi, int radius, int blocks, cudaStream_t stream);
+const void *dnls_stencil_kernel_ptr(int radius, bool team, bool windowed = false);
+// dynamic shared memory of a block: `len` sites (a chain, or a window) on `lanes` lanes
+size_t dnls_stencil_smem(uint32_t len, int lanes, int radius);
 cudaError_t launch_dnls_nonlinear(double2 *psi, uint64_t elements, double coef, const double2 *sctab,
                                   cudaStream_t stream);
 cudaError_t launch_dnls_linear(double2 *psi, uint64_t elements, uint32_t n, const double2 *table,

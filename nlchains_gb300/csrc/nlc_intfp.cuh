@@ -45,14 +45,13 @@ __device__ __forceinline__ uint64_t mad_wide(uint32_t a, uint32_t b, uint64_t c)
 __device__ __forceinline__ uint32_t lo32(uint64_t a) { return uint32_t(a); }
 __device__ __forceinline__ uint32_t hi32(uint64_t a) { return uint32_t(a >> 32); }
 
-// a - b.  Both significands are placed with the leading bit at bit 61 of 64 (carry at 62, sign at
+// a + b, the high word of b given apart (int_sub flips its sign).  Both significands are placed with the leading bit at bit 61 of 64 (carry at 62, sign at
 // 63), 9 bits below the last one kept; the smaller operand is shifted right, its lost bits ORed
 // into its lowest one, and added or (two's complement) subtracted; the sum's leading bit goes to
 // bit 62 and the 10 bits below the 53 kept are rounded off.  The hidden bit is added into the
 // exponent field, which also takes the carry of the rounding.
-__device__ __forceinline__ double int_sub(double a, double b, IntFlags &f) {
-	const uint32_t ah = __double2hiint(a), al = __double2loint(a), bh = __double2hiint(b) ^ 0x80000000u,
-	               bl = __double2loint(b);
+__device__ __forceinline__ double int_add_words(double a, uint32_t bh, uint32_t bl, IntFlags &f) {
+	const uint32_t ah = __double2hiint(a), al = __double2loint(a);
 	const uint32_t aa = ah & 0x7fffffffu, ba = bh & 0x7fffffffu;
 	const bool swap = aa < ba;   // by the high words: equal ones cancel and are flagged where it matters
 	const uint32_t xh = swap ? bh : ah, xl = swap ? bl : al, yl = al + bl - xl;
@@ -77,6 +76,36 @@ __device__ __forceinline__ double int_sub(double a, double b, IntFlags &f) {
 	f.exmax = max(f.exmax, ex - 64u);
 	f.rmin = min(f.rmin, int32_t(rh));
 	return __hiloint2double(int(((oh >> 10) + (ex - s) * 0x100000u) | (xh & 0x80000000u)), int(__funnelshift_r(ol, oh, 10)));
+}
+
+__device__ __forceinline__ double int_add(double a, double b, IntFlags &f) {
+	return int_add_words(a, __double2hiint(b), __double2loint(b), f);
+}
+__device__ __forceinline__ double int_sub(double a, double b, IntFlags &f) {
+	return int_add_words(a, __double2hiint(b) ^ 0x80000000u, __double2loint(b), f);
+}
+
+// a b: the exact product of the 53-bit significands, leading bit at 104 or 105 of 128, the low 32 bits
+// ORed into the rounding as one.
+__device__ __forceinline__ double int_mul(double a, double b, IntFlags &f) {
+	const uint32_t ah = __double2hiint(a), a0 = __double2loint(a), bh = __double2hiint(b), b0 = __double2loint(b);
+	const uint32_t a1 = (ah & 0xfffffu) | 0x100000u, b1 = (bh & 0xfffffu) | 0x100000u;
+	const uint32_t ea = (ah >> 20) & 0x7ffu, eb = (bh >> 20) & 0x7ffu;
+	const uint64_t low = mul_wide(a0, b0);
+	const uint64_t mid = mad_wide(a0, b1, mad_wide(a1, b0, uint64_t(hi32(low))));
+	const uint64_t top = mad_wide(a1, b1, uint64_t(hi32(mid)));   // the product's bits from 64 on
+	const uint32_t carry = hi32(top) >> 9;                        // 1: leading bit at 105
+	// the 53 bits kept in (w2, w1), the rest in w0 with its first bit at bit 31
+	const uint32_t up = 0x1000u >> carry;
+	const uint64_t u0 = mul_wide(lo32(mid), up), u1 = mul_wide(lo32(top), up);
+	const uint32_t w0 = lo32(u0) | min(lo32(low), 1u), w1 = lo32(u1) + hi32(u0), w2 = hi32(top) * up + hi32(u1);
+	// to nearest, ties to even: up where w0, its lowest bit replaced by w1's at a tie, exceeds 2^31
+	const uint32_t inc = (w0 | (w1 & 1u)) > 0x80000000u ? 1u : 0u;
+	uint32_t ol, oh;
+	asm("{add.cc.u32 %0, %2, %3; addc.u32 %1, %4, 0;}" : "=r"(ol), "=r"(oh) : "r"(w1), "r"(inc), "r"(w2));
+	const uint32_t e = ea + eb + carry;   // result exponent + 1023, less the hidden bit's 1 below
+	f.exmax = max(max(f.exmax, ea - 64u), max(eb - 64u, e - 1088u));
+	return __hiloint2double(int((oh + (e - 1024u) * 0x100000u) ^ ((ah ^ bh) & 0x80000000u)), int(ol));
 }
 
 // An addend K > 0 of int_square_plus: its significand with the leading bit at bit 62 of 64, its

@@ -124,7 +124,7 @@ struct nlc_plan {
 	size_t dnls_smem = 0;
 	DnlsStencilArgs sa{};      // DNLS in the real-space stencil form (tier 5)
 	bool dnls_stencil = false;
-	int dnls_sites = 0, dnls_radius = 0;
+	int dnls_lanes = 0, dnls_sites = 0, dnls_radius = 0;
 	DiagArgs ga{};
 	int diag_blocks = 0, diag_threads = 0, diag_team_block = 0, diag_rows = 0;
 	size_t diag_smem = 0;
@@ -724,11 +724,9 @@ static uint32_t dnls_window_steps(uint32_t win_len, int radius) {
 	return std::max<uint32_t>(1, win_len / (140 * uint32_t(radius)));
 }
 
-// DNLS in the real-space stencil form (nlc_dnls_stencil.cu), where it applies: the propagator's
-// taps beyond radius 11 below 2^-64 (dt d_k up to ~0.05), n >= 2R + 2, and a launch shape of G lanes
-// (up to 256) of E or E - 1 sites, E in {16, 12, 8} with E - 1 >= R.  Among the shapes, the one
-// with the fewest lane-sites computed per chain site (idle lanes of a warp, the short lanes' inert
-// slot); otherwise P.dnls_stencil stays false and the plan takes the Fourier form.
+// DNLS in the real-space stencil form (nlc_dnls_stencil.cu), where it applies: the propagator's taps
+// beyond radius 11 below 2^-64 (dt d_k up to ~0.05) and n >= 2R + 2; otherwise P.dnls_stencil stays false
+// and the plan takes the Fourier form.
 static int setup_dnls_stencil(nlc_plan &P) {
 	const uint32_t n = P.m.chain_length;
 	DnlsStencilArgs &a = P.sa;
@@ -736,20 +734,28 @@ static int setup_dnls_stencil(nlc_plan &P) {
 	const int R = need <= 7 ? 7 : need <= kMaxStencilRadius ? kMaxStencilRadius : 0;
 	if (!R || n < uint32_t(2 * R + 2)) return NLC_OK;
 	int lanes = 0, sites = 0;
-	double best = 0;
 	// NLC_DNLS_SITES=<E> restricts the shapes to E sites per lane (used by the tests to cover every
 	// instantiation); NLC_FORCE_WINDOW=<G> integrates in windows of G lanes where a block would hold
 	// the chain (used by the tests to cover the windowed form on short chains)
 	int only = 0;
 	if (const char *e = std::getenv("NLC_DNLS_SITES")) only = std::atoi(e);
 	const char *force_win = std::getenv("NLC_FORCE_WINDOW");
-	for (int E : {16, 12, 8}) {
-		if (force_win || E - 1 < R || (only && E != only)) continue;
+	// The lanes take the sites row by row.  A scheduler with one warp of the ensemble runs a row in ~2900
+	// clocks (R = 7: the integer and the FP64 work of a warp hardly overlap), one with several a row
+	// of each in ~1900 (the FP64 pipe): the sites per lane with the least of rows x that, G as few
+	// lanes (up to 256) as hold the chain in so many rows.  Few chains get one site per lane (96 chains of
+	// 24 sites: 5 steps in 0.07 ms, 0.91 with 12), a full GPU 8 (16 leave half the warps, within 3%);
+	// 12 only where the others leave over 4% more lanes idle.
+	double least = 0, least_sites = 0;   // lane-sites computed per chain
+	for (int E : {8, 16, 4, 2, 1, 12}) {
+		if (force_win || (only && E != only)) continue;
 		// G (E - 1) < n <= G E: every lane holds E or E - 1 sites
 		for (uint32_t G = (n + E - 1) / E; G <= 256 && uint64_t(G) * (E - 1) < n; G++) {
-			const double occupied = G <= 32 ? 32. / double(32 / G) : double((G + 31) / 32 * 32);
-			const double eff = double(n) / (occupied * E);
-			if (eff > best * 1.0001) best = eff, lanes = int(G), sites = E;
+			const double warps = G <= 32 ? std::ceil(double(P.m.copies) / (32 / G)) : double(P.m.copies) * ((G + 31) / 32);
+			const double lane_sites = E * (G <= 32 ? 32. / double(32 / G) : double((G + 31) / 32 * 32));
+			const double cost = E * std::max(2900., 1900. * warps / (4. * P.prop.multiProcessorCount));
+			if (!lanes || (E == 12 ? lane_sites < 0.96 * least_sites && cost < least : cost < 0.97 * least))
+				least = cost, least_sites = lane_sites, lanes = int(G), sites = E;
 		}
 	}
 	bool windowed = false;
@@ -760,18 +766,18 @@ static int setup_dnls_stencil(nlc_plan &P) {
 		// (window minus 7 R s sites at each end, s = dnls_window_steps) tiling the chain
 		int G = force_win ? std::atoi(force_win) : 0;
 		if (!G) {
-			uint64_t least = ~0ull;
+			uint64_t least_work = ~0ull;
 			for (int g = 256; g >= 64; g -= 32) {
 				const uint32_t len = uint32_t(g) * 16, halo = 7 * uint32_t(R) * dnls_window_steps(len, R);
 				if (len >= n || 2 * halo >= len) continue;
 				const uint64_t work = uint64_t((n + len - 2 * halo - 1) / (len - 2 * halo)) * len;
-				if (work < least) least = work, G = g;
+				if (work < least_work) least_work = work, G = g;
 			}
 		}
 		if (G <= 32 || G > 256 || G % 32 || uint64_t(G) * 16 >= n) return NLC_OK;
 		lanes = G, sites = 16, windowed = true;
 	}
-	const void *k = dnls_stencil_kernel_ptr(sites, R, lanes <= 32, windowed);
+	const void *k = dnls_stencil_kernel_ptr(R, lanes <= 32, windowed);
 	if (!k) return NLC_OK;
 	const DnlsArgs &d = P.da;
 	a.n = n, a.copies = P.m.copies, a.lanes = lanes;
@@ -780,8 +786,19 @@ static int setup_dnls_stencil(nlc_plan &P) {
 	a.work_counter = P.d_counter;
 	a.sctab = d.sctab;
 	P.dnls_threads = lanes <= 32 ? 128 : (lanes + 31) / 32 * 32;
-	P.dnls_smem = dnls_stencil_smem(lanes, R);
+	if (windowed) {
+		// a window's rows run over a block of 256 to 384 threads, the width that leaves the fewest idle
+		// (of the last row), so that the few windows of a small ensemble do not serialise on few warps
+		const uint32_t len = uint32_t(lanes) * sites;
+		uint32_t idle = ~0u;
+		for (uint32_t t = 384; t >= 256; t -= 32)
+			if ((len + t - 1) / t * t - len < idle) idle = (len + t - 1) / t * t - len, P.dnls_threads = int(t);
+		a.lanes = P.dnls_threads;
+	}
+	P.dnls_lanes = lanes;
+	P.dnls_smem = dnls_stencil_smem(windowed ? uint32_t(lanes) * sites : n, lanes, R);
 	int per_sm = 0, rc;
+	if ((rc = set_smem_attr(k, P.dnls_smem, P.prop))) return rc;
 	if ((rc = cuda_status(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, P.dnls_threads, P.dnls_smem),
 	                      "occupancy")))
 		return rc;
@@ -800,8 +817,9 @@ static int setup_dnls_stencil(nlc_plan &P) {
 	}
 	P.dnls_sites = sites, P.dnls_radius = R;
 	P.dnls_stencil = true;
-	// a block's step: 7 sub-steps of 19 + 4R FP64 operations on the lane-sites it computes, at ~85%
-	P.block_ops = 7. * (19 + 4 * R) * double(sites) * (lanes <= 32 ? 32 * (P.dnls_threads / 32) : P.dnls_threads) / 0.85;
+	// a block's step: 7 sub-steps of 19 + 4R operations on the lane-sites it computes, at ~1.4 of the FP64
+	// rate (a part of them runs on the integer pipes)
+	P.block_ops = 7. * (19 + 4 * R) * (windowed ? double(lanes) * sites : double(sites) * P.dnls_threads) / 1.4;
 	P.per_sm = per_sm;
 	P.block_warps = P.dnls_threads / 32;
 	P.tier = windowed ? 6 : 5;
@@ -1084,7 +1102,7 @@ void nlc::plan_destroy_ordered(nlc_plan *plan, cudaStream_t stream) {
 extern "C" int nlc_plan_shape(const nlc_plan *P, int32_t *lanes, int32_t *sites, int32_t *threads, int32_t *tier) {
 	if (!P) return set_error(NLC_EINVAL, "plan is NULL");
 	if (P->m.model == NLC_DNLS && P->dnls_stencil) {
-		if (lanes) *lanes = P->sa.lanes;
+		if (lanes) *lanes = P->dnls_lanes;
 		if (sites) *sites = P->dnls_sites;
 		if (threads) *threads = P->dnls_threads;
 		if (tier) *tier = P->tier;
@@ -1260,7 +1278,7 @@ int nlc::move_segment(nlc_plan *P, void *state, uint32_t steps, uint32_t seg, cu
 			const unsigned long long units = (unsigned long long) P->m.copies * a.win_count;
 			const int blocks = int(std::min<unsigned long long>(
 			    units, (P->m.flags & NLC_FLAG_SHARED_GPU) ? 0x7fffffffull : (unsigned long long) P->dnls_blocks));
-			int rc = cuda_status(launch_dnls_stencil(a, in, P->dnls_sites, P->dnls_radius, blocks, st),
+			int rc = cuda_status(launch_dnls_stencil(a, in, P->dnls_radius, blocks, st),
 			                     "DNLS windowed stencil launch");
 			if (rc) return rc;
 			std::swap(in, out);
@@ -1276,8 +1294,7 @@ int nlc::move_segment(nlc_plan *P, void *state, uint32_t steps, uint32_t seg, cu
 		DnlsStencilArgs a = P->sa;
 		a.steps = steps;
 		a.seg = seg;
-		return cuda_status(launch_dnls_stencil(a, static_cast<double2 *>(state), P->dnls_sites, P->dnls_radius,
-		                                       P->dnls_blocks, st),
+		return cuda_status(launch_dnls_stencil(a, static_cast<double2 *>(state), P->dnls_radius, P->dnls_blocks, st),
 		                   "DNLS stencil move launch");
 	}
 	if (P->m.model == NLC_DNLS) {

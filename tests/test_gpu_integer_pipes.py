@@ -68,3 +68,32 @@ def test_bits_at_edge_operands(gpu, monkeypatch, model, params, n, lanes):
     assert np.array_equal(finite, np.isfinite(out))
     bad = (out.view(np.uint64) != exp.view(np.uint64)) & finite
     assert not bad.any(), f"rows {np.unique(np.nonzero(bad)[0])}: {np.count_nonzero(bad)} values differ"
+
+
+# sites per lane 1 .. 16 (rows over several chains of a warp, one chain of a warp, a block), both radii, and windows
+@pytest.mark.parametrize("n,dt,sites,window", [(16, 0.01, 0, 0), (33, 0.01, 1, 0), (64, 0.01, 2, 0), (24, 0.05, 12, 0),
+                                               (100, 0.05, 8, 0), (250, 0.01, 1, 0), (515, 0.01, 16, 0),
+                                               (1021, 0.05, 4, 0), (1300, 0.01, 0, 64), (2100, 0.05, 0, 96)])
+def test_dnls_bits_at_edge_operands(gpu, monkeypatch, n, dt, sites, window):
+    """The DNLS stencil form on the same states (phi + i pi as psi: real, imaginary and zero sites, angles on
+    both sides of 2^-4 within a warp)."""
+    if sites:
+        monkeypatch.setenv("NLC_DNLS_SITES", str(sites))
+    if window:
+        monkeypatch.setenv("NLC_FORCE_WINDOW", str(window))
+    state = edge_states(n, n)
+    copies, steps = len(state), 2
+    shape = gpu.Plan(gpu.Model("DNLS", n, copies, dt, beta=1.0)).shape()
+    assert shape["tier"] == (6 if window else 5) and (not sites or shape["sites_per_lane"] == sites)
+    ctx = gpu.Context(0)
+    job = ctx.job(gpu.Model("DNLS", n, copies, dt, beta=1.0), steps)
+    job.upload(state)
+    job.advance(2 * steps)
+    out = job.download()
+    job.close()
+    ctx.close()
+    exp = O.advance(O.Model("DNLS", n, copies, dt, beta=1.0), state, 2 * steps, steps, order=O.ORDER_STENCIL)
+    exp = exp.reshape(copies, n, 2)
+    assert np.isfinite(exp).all()
+    bad = out.view(np.uint64) != exp.view(np.uint64)
+    assert not bad.any(), f"rows {np.unique(np.nonzero(bad)[0])}: {np.count_nonzero(bad)} values differ"
