@@ -42,6 +42,13 @@ __device__ __forceinline__ FpOnes in_register(const FpOnes &k, int zero) {
 	r.one = in_register(k.one, zero), r.mone = in_register(k.mone, zero), r.mzero = in_register(k.mzero, zero);
 	return r;
 }
+__device__ __forceinline__ ExpConsts in_register(const ExpConsts &c, int zero) {
+	ExpConsts r;
+	r.shifter = in_register(c.shifter, zero), r.inv_l = in_register(c.inv_l, zero);
+	r.l1 = in_register(c.l1, zero), r.l2 = in_register(c.l2, zero);
+	r.c3 = in_register(c.c3, zero), r.c2 = in_register(c.c2, zero);
+	return r;
+}
 // the constants of sincos_table's small-angle series (the others, of its table branch, stay where
 // they are: most angles are small)
 __device__ __forceinline__ SinCosConsts in_register(const SinCosConsts &c, int zero) {

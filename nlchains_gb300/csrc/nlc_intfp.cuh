@@ -18,6 +18,7 @@
 #include <cstdint>
 #include <cuda_runtime.h>
 
+#include "nlc_device.cuh"
 #include "nlc_internal.h"
 
 namespace nlc {
@@ -141,6 +142,33 @@ __device__ __forceinline__ double int_square_plus(double c, const IntAddend &K, 
 	const uint32_t top = oh >> drop;                                     // 0 where the rounding wrapped
 	f.rmin = min(f.rmin, min(s, int32_t(top)));
 	return __hiloint2double(int(top + K.field + carry * 0x100000u), int(__funnelshift_r(ol, oh, drop)));
+}
+
+// n as a double, |n| < 2^24: through its FP32 value, exact, whose exponent and significand are moved to the
+// double's places.
+__device__ __forceinline__ double int_to_double(int n) {
+	const uint32_t b = __float_as_uint(float(n));
+	const uint32_t h = ((b & 0x7fffffffu) >> 3) + 0x38000000u;
+	return __hiloint2double(int(n ? h | (b & 0x80000000u) : 0u), int(b << 29));
+}
+
+// exp_scaled (nlc_device.cuh) with the table index's value and the product of the polynomial on the
+// integer pipes: 6 of its 8 operations stay on the FP64 pipe.  Flagged where exp_scaled leaves its fast
+// path, and somewhat before.
+__device__ __forceinline__ double exp_scaled_mixed(double x, const double *__restrict__ table, const FpOnes &k1,
+                                                   const ExpConsts &c, IntFlags &f) {
+	f.rmin = min(f.rmin, 0x40b00000 - (__double2hiint(x) & 0x7fffffff));   // |x| < 4096: |n| < 2^24
+	const int n = __double2loint(dfma(x, c.inv_l, c.shifter));
+	const double nf = int_to_double(n);
+	double r = dfma(-nf, c.l1, x);
+	r = dfma(-nf, c.l2, r);
+	double q = dfma(r, c.c3, c.c2);
+	q = dfma(q, r, k1.one);
+	const double tj = table[n & (kExpTable - 1)];
+	const double v = dfma(tj, int_mul(q, r, f), tj);
+	const int k = n >> 11, hi = __double2hiint(v);
+	f.exmax = max(f.exmax, uint32_t(((hi >> 20) & 0x7ff) + k - 64));
+	return __hiloint2double(hi + k * 0x100000, __double2loint(v));
 }
 
 }  // namespace nlc

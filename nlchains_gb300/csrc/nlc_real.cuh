@@ -101,17 +101,32 @@ struct Ring {
 	}
 };
 
+struct ForceConsts {
+	double alpha, beta, alpha2, mp2;
+	ExpConsts ek;
+};
+
 // Bond force term V'(d) of the bond-based models.
 template <int MODEL, int VAR>
-__device__ __forceinline__ double bond_force(double d, const RealArgs &a, const double *tab) {
+__device__ __forceinline__ double bond_force(double d, const ForceConsts &c, const FpOnes &k1, const double *tab) {
 	if constexpr (MODEL == NLC_FPUT) {
 		// d + alpha d^2 + beta d^3 = d * (1 + d * (alpha + beta d))
-		const double h = VAR ? d : dfma(a.beta, d, a.alpha);
-		const double w = dfma(h, d, a.k1.one);
-		return fmul(d, w, a.k1);
+		const double h = VAR ? d : dfma(c.beta, d, c.alpha);
+		return fmul(d, dfma(h, d, k1.one), k1);
 	} else {
 		// (exp(2 alpha d) - 1) / (2 alpha) up to the constant, which cancels in g[s] - g[s-1]
-		return exp_scaled(VAR ? d : fmul(a.alpha2, d, a.k1), tab, a.k1, a.ek);
+		return exp_scaled(VAR ? d : fmul(c.alpha2, d, k1), tab, k1, c.ek);
+	}
+}
+// the same with its products on the integer pipes
+template <int MODEL, int VAR>
+__device__ __forceinline__ double bond_force_mixed(double d, const ForceConsts &c, const FpOnes &k1, const double *tab,
+                                                   IntFlags &f) {
+	if constexpr (MODEL == NLC_FPUT) {
+		const double h = VAR ? d : dfma(c.beta, d, c.alpha);
+		return int_mul(d, dfma(h, d, k1.one), f);
+	} else {
+		return exp_scaled_mixed(VAR ? d : int_mul(c.alpha2, d, f), tab, k1, c.ek, f);
 	}
 }
 
@@ -159,6 +174,12 @@ __global__ void real_move_kernel_t(double2 *__restrict__ state, const RealArgs a
 	const int gpb = blockDim.x / G;          // groups per block
 
 	Ring ring{G, lane, tid & 31, tid >> 5, G > 32 ? G >> 5 : 1, xbuf, 0};
+
+	// the constants and, per sub-step, the coefficients as vector-register operands (nlc_device.cuh)
+	const int zero = lane_zero(a.k1);
+	const FpOnes k1 = in_register(a.k1, zero);
+	const ForceConsts fc{in_register(a.alpha, zero), in_register(a.beta, zero), in_register(a.alpha2, zero),
+	                     in_register(a.mp2, zero), in_register(a.ek, zero)};
 
 	if constexpr (MODEL == NLC_TODA) {
 		for (int i = tid; i < kExpTable; i += blockDim.x) s_tab[i] = a.exptab[i];
@@ -271,67 +292,91 @@ __global__ void real_move_kernel_t(double2 *__restrict__ state, const RealArgs a
 #pragma unroll (INT ? 1 : 7)
 			for (int k = 0; k < 7; k++) {
 				// the trailing drift of step i-1 (c[7]) merged with the leading drift of step i (c[0])
-				const double cd = k == 0 ? (i == 0 ? cd_lead : boundary ? a.cd[0] : a.cd0_merged) : a.cd[k];
+				const double cd = in_register(k == 0 ? (i == 0 ? cd_lead : boundary ? a.cd[0] : a.cd0_merged) : a.cd[k], zero);
+				constexpr bool kOnSite = MODEL == NLC_DNKG || MODEL == NLC_DDNKG;
+				const double ck = in_register(kOnSite ? a.nck[k] : a.ck[k], zero);
 #pragma unroll
 				for (int j = 0; j < E; j++) x[j + 1] = dfma(cd, p[j], x[j + 1]);
 
-				if constexpr (MODEL == NLC_DNKG || MODEL == NLC_DDNKG) {
+				if constexpr (kOnSite) {
 					double l, r;
 					ring.template both<SHFL>(fl ? x[E] : x[E - 1], x[1], l, r);
 					x[0] = l, x[E + 1] = r;
 					if (!fl) x[E] = r;
 					auto mp2 = [&](int j) {
 						if constexpr (MODEL == NLC_DDNKG) return mv[j - 1];
-						else return a.mp2;
+						else return fc.mp2;
 					};
 					auto force_fp64 = [&](int j) {
 						const double c = x[j];
-						const double bc = VAR ? c : fmul(a.beta, c, a.k1);
-						return fsub(dfma(c, dfma(bc, c, mp2(j)), -x[j - 1]), x[j + 1], a.k1);
+						const double bc = VAR ? c : fmul(fc.beta, c, k1);
+						return fsub(dfma(c, dfma(bc, c, mp2(j)), -x[j - 1]), x[j + 1], k1);
 					};
 					if constexpr (!INT) {
 #pragma unroll
-						for (int j = 1; j <= E; j++) p[j - 1] = dfma(a.nck[k], force_fp64(j), p[j - 1]);
+						for (int j = 1; j <= E; j++) p[j - 1] = dfma(ck, force_fp64(j), p[j - 1]);
 					} else {
-						// the square (beta = 1) and the subtraction on the integer pipes, a batch at a time
+						// the subtraction and the square (beta = 1) or the product beta x (beta != 0, else every
+						// one would be flagged) on the integer pipes, a batch at a time
+						auto kick = [&](auto beta_tag) {
 #pragma unroll
-						for (int j0 = 1; j0 <= E; j0 += kIntBatch) {
-							IntFlags f, fe;
-							double v[kIntBatch];
+							for (int j0 = 1; j0 <= E; j0 += kIntBatch) {
+								IntFlags f, fe;
+								double v[kIntBatch];
 #pragma unroll
-							for (int j = j0; j <= E && j < j0 + kIntBatch; j++) {
-								IntFlags &fj = j == E ? fe : f;
-								const double c = x[j];
-								double t;
-								if constexpr (!VAR) {
-									t = dfma(fmul(a.beta, c, a.k1), c, mp2(j));
-								} else if constexpr (MODEL == NLC_DDNKG) {
-									t = int_square_plus(c, int_addend(mv[j - 1]), fj);
-								} else {
-									t = int_square_plus(c, a.mp2_int, fj);
+								for (int j = j0; j <= E && j < j0 + kIntBatch; j++) {
+									IntFlags &fj = j == E ? fe : f;
+									const double c = x[j];
+									double t;
+									if constexpr (!VAR) {
+										if constexpr (decltype(beta_tag)::value) t = dfma(int_mul(fc.beta, c, fj), c, mp2(j));
+										else t = dfma(fmul(fc.beta, c, k1), c, mp2(j));
+									} else if constexpr (MODEL == NLC_DDNKG) {
+										t = int_square_plus(c, int_addend(mv[j - 1]), fj);
+									} else {
+										t = int_square_plus(c, a.mp2_int, fj);
+									}
+									v[j - j0] = int_sub(dfma(c, t, -x[j - 1]), x[j + 1], fj);
 								}
-								v[j - j0] = int_sub(dfma(c, t, -x[j - 1]), x[j + 1], fj);
-							}
-							if (__any_sync(0xffffffffu, mv_bad | f.bad() | (fl & fe.bad()))) {
+								if (__any_sync(0xffffffffu, mv_bad | f.bad() | (fl & fe.bad()))) {
 #pragma unroll
-								for (int j = j0; j <= E && j < j0 + kIntBatch; j++) v[j - j0] = force_fp64(j);
-							}
+									for (int j = j0; j <= E && j < j0 + kIntBatch; j++) v[j - j0] = force_fp64(j);
+								}
 #pragma unroll
-							for (int j = j0; j <= E && j < j0 + kIntBatch; j++) p[j - 1] = dfma(a.nck[k], v[j - j0], p[j - 1]);
-						}
+								for (int j = j0; j <= E && j < j0 + kIntBatch; j++) p[j - 1] = dfma(ck, v[j - j0], p[j - 1]);
+							}
+						};
+						if (VAR || a.beta != 0.) kick(std::true_type{});
+						else kick(std::false_type{});
 					}
 				} else {
 					const double r = ring.template from_right<SHFL>(x[1]);
 					x[E + 1] = r;
 					if (!fl) x[E] = r;
 					double g[E + 1], d[E];
-					sub_batch<E, INT>(d, x + 2, x + 1, fl, a.k1);
+					if constexpr (!INT) {
 #pragma unroll
-					for (int j = 1; j <= E; j++) g[j] = bond_force<MODEL, VAR>(d[j - 1], a, s_tab);
+						for (int j = 1; j <= E; j++) g[j] = bond_force<MODEL, VAR>(fsub(x[j + 1], x[j], k1), fc, k1, s_tab);
+					} else {
+#pragma unroll
+						for (int j0 = 1; j0 <= E; j0 += kIntBatch) {
+							IntFlags f, fe;
+#pragma unroll
+							for (int j = j0; j <= E && j < j0 + kIntBatch; j++) {
+								IntFlags &fj = j == E ? fe : f;
+								g[j] = bond_force_mixed<MODEL, VAR>(int_sub(x[j + 1], x[j], fj), fc, k1, s_tab, fj);
+							}
+							if (__any_sync(0xffffffffu, f.bad() | (fl & fe.bad()))) {
+#pragma unroll
+								for (int j = j0; j <= E && j < j0 + kIntBatch; j++)
+									g[j] = bond_force<MODEL, VAR>(fsub(x[j + 1], x[j], k1), fc, k1, s_tab);
+							}
+						}
+					}
 					g[0] = ring.template from_left<SHFL>(fl ? g[E] : g[E - 1]);
-					sub_batch<E, INT>(d, g + 1, g, fl, a.k1);
+					sub_batch<E, INT>(d, g + 1, g, fl, k1);
 #pragma unroll
-					for (int j = 0; j < E; j++) p[j] = dfma(a.ck[k], d[j], p[j]);
+					for (int j = 0; j < E; j++) p[j] = dfma(ck, d[j], p[j]);
 				}
 				if (!fl) p[E - 1] = 0.;   // the slot past a short lane's last site stays inert
 			}
