@@ -75,8 +75,8 @@ enum {
 	                                    global-memory passes keep the FP64 diagnostics */
 	NLC_FLAG_DNLS_FOURIER = 512      /* DNLS: the linear sub-steps through transforms of the chain, as
 	                                    the reference does, at every length.  By default, where dt is
-	                                    small enough (propagator taps beyond 11 sites below 2^-64, dt up
-	                                    to ~0.05) and chain_length >= 2R + 2 (16 at dt = 0.01), each
+	                                    small enough (propagator taps beyond 13 sites below 2^-64, dt up
+	                                    to ~0.15) and chain_length >= 2R + 2 (16 at dt = 0.01), each
 	                                    linear sub-step is the same operator applied as its real-space
 	                                    stencil (nlc_dnls_stencil_coefficients) */
 };

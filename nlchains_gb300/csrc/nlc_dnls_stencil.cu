@@ -55,20 +55,32 @@ __device__ __forceinline__ double2 rotate_phase(double2 v, double neg_coef, doub
 	return make_double2(dfma(v.x, c, -fmul(v.y, s, k)), dfma(v.x, s, fmul(v.y, c, k)));
 }
 
-// The same with the products of two varying factors on the integer pipes (5 of the 17 operations of an
-// angle below 2^-4); redone by rotate_phase where a lane's operands ask for it.  Every lane of the
-// warp calls it.
+// The same with the products of two varying factors on the integer pipes: 5 of the 17 operations of an
+// angle below 2^-4, 6 of the 21 of the table method, in warps whose angles are all of one kind (mixed
+// ones take sincos_table as it is); redone by rotate_phase where a lane's operands ask for it.  Every
+// lane of the warp calls it.
 __device__ __forceinline__ double2 rotate_phase_mixed(double2 v, double neg_coef, double neg_phase,
                                                       const double2 *__restrict__ sctab, const SinCosConsts &C,
                                                       const FpOnes &k) {
 	IntFlags f;
 	const double th = dfma(neg_coef, dfma(v.x, v.x, int_mul(v.y, v.y, f)), neg_phase);
+	const int hi = __double2hiint(th) & 0x7fffffff;
 	double s, c;
-	if (__all_sync(0xffffffffu, (__double2hiint(th) & 0x7fffffff) < 0x3fb00000)) {   // sincos_table's series
+	if (__all_sync(0xffffffffu, hi < 0x3fb00000)) {   // sincos_table's series
 		const double t2 = int_mul(th, th, f);
 		const double ps = dfma(t2, dfma(t2, dfma(t2, C.q9, C.q7), C.q5), C.q3);
 		s = dfma(int_mul(th, t2, f), ps, th);
 		c = dfma(t2, dfma(t2, dfma(t2, dfma(t2, C.w8, C.w6), C.w4), C.w2), k.one);
+	} else if (__all_sync(0xffffffffu, hi >= 0x3fb00000 && hi < 0x41300000)) {   // sincos_table's table
+		const double t = dfma(th, C.inv, C.shifter);
+		const double kd = fsub(t, C.shifter, k);
+		const double r = dfma(-kd, C.p2, dfma(-kd, C.p1, th));
+		const double2 e = __ldg(sctab + (__double2loint(t) & (kSinCosTable - 1)));
+		const double r2 = int_mul(r, r, f);
+		const double sr = dfma(int_mul(r, r2, f), dfma(r2, C.s5, C.s3), r);
+		const double cm1 = int_mul(r2, dfma(r2, C.c4, C.c2), f);
+		c = dfma(e.x, cm1, dfma(-e.y, sr, e.x));
+		s = dfma(e.y, cm1, dfma(e.x, sr, e.y));
 	} else {
 		sincos_table(th, sctab, C, k, &s, &c);
 	}
@@ -81,21 +93,25 @@ __device__ __forceinline__ double2 rotate_phase_mixed(double2 v, double neg_coef
 // One component (the real or the imaginary part) of the (2R + 1)-point stencil at one site:
 // psi + (J_0 - 1) psi + sum_x J_x i^x (psi_{s+x} + psi_{s-x}).  `own` and `other` point at the site's
 // component and its counterpart; the factor i of odd x takes the sums from `other`, and the taps carry
-// the signs.  `add` forms the sums.
-template <int R, class Add>
-__device__ __forceinline__ double stencil_component(const double *own, const double *other, const double *tp, Add add) {
+// the signs.  `near` forms the sums up to kIntTaps sites away, `far` those beyond: at radius 13 the
+// integer pipes would otherwise have as much to do as the FP64 pipe (n = 500, 1024 chains, dt = 0.1, 10
+// steps: 3.98 ms with the sums up to 4 on the integer pipes, 3.58 up to 9, 3.92 with all 13).
+constexpr int kIntTaps = 10;
+template <int R, class Near, class Far>
+__device__ __forceinline__ double stencil_component(const double *own, const double *other, const double *tp, Near near,
+                                                    Far far) {
 	double y = dfma(tp[0], own[0], own[0]);
 #pragma unroll
 	for (int x = 1; x <= R; x++) {
 		const double *w = x & 1 ? other : own;
-		y = dfma(tp[x], add(w[x], w[-x]), y);
+		y = dfma(tp[x], x <= kIntTaps ? near(w[x], w[-x]) : far(w[x], w[-x]), y);
 	}
 	return y;
 }
 
 // double2s of the constants ahead of the buffers: the taps, the rotations, the sine and cosine series
 template <int R>
-constexpr int kStencilConsts = 7 * (R + 1) + 9 + 4;
+constexpr int kStencilConsts = 7 * (R + 1) + 9 + 8;
 
 // TEAM: G <= 32, 128-thread blocks; otherwise one chain (WIN: one window) per block of ceil(G / 32)
 // warps
@@ -136,13 +152,17 @@ __global__ void __launch_bounds__(TEAM ? 128 : WIN ? 384 : 256, WIN ? 2 : (TEAM 
 	if (tid == 0) {
 		ser_sm[0] = a.sc.q3, ser_sm[1] = a.sc.q5, ser_sm[2] = a.sc.q7, ser_sm[3] = a.sc.q9;
 		ser_sm[4] = a.sc.w2, ser_sm[5] = a.sc.w4, ser_sm[6] = a.sc.w6, ser_sm[7] = a.sc.w8;
+		ser_sm[8] = a.sc.shifter, ser_sm[9] = a.sc.inv, ser_sm[10] = a.sc.p1, ser_sm[11] = a.sc.p2;
+		ser_sm[12] = a.sc.s3, ser_sm[13] = a.sc.s5, ser_sm[14] = a.sc.c2, ser_sm[15] = a.sc.c4;
 	}
 	const int zero = lane_zero(a.k1);
 	const FpOnes k1 = in_register(a.k1, zero);
 	auto rotate = [&](double2 v, int i) {
-		SinCosConsts sc = a.sc;
+		SinCosConsts sc;
 		sc.q3 = ser_sm[0], sc.q5 = ser_sm[1], sc.q7 = ser_sm[2], sc.q9 = ser_sm[3];
 		sc.w2 = ser_sm[4], sc.w4 = ser_sm[5], sc.w6 = ser_sm[6], sc.w8 = ser_sm[7];
+		sc.shifter = ser_sm[8], sc.inv = ser_sm[9], sc.p1 = ser_sm[10], sc.p2 = ser_sm[11];
+		sc.s3 = ser_sm[12], sc.s5 = ser_sm[13], sc.c2 = ser_sm[14], sc.c4 = ser_sm[15];
 		const double2 c = rot_sm[i];
 		return rotate_phase_mixed(v, c.x, c.y, a.sctab, sc, k1);
 	};
@@ -206,9 +226,10 @@ __global__ void __launch_bounds__(TEAM ? 128 : WIN ? 384 : 256, WIN ? 2 : (TEAM 
 					const double *own = w + c * pitch, *other = w + (1 - c) * pitch, *t = tp + c * (R + 1);
 					// the sums on the integer pipes; redone on the FP64 pipe where a lane's operands ask for it
 					IntFlags f;
-					double v = stencil_component<R>(own, other, t, [&](double u, double v) { return int_add(u, v, f); });
-					if (__any_sync(0xffffffffu, f.bad()))
-						v = stencil_component<R>(own, other, t, [&](double u, double v) { return fadd(u, v, k1); });
+					auto int_sum = [&](double u, double v) { return int_add(u, v, f); };
+					auto fp64_sum = [&](double u, double v) { return fadd(u, v, k1); };
+					double v = stencil_component<R>(own, other, t, int_sum, fp64_sum);
+					if (__any_sync(0xffffffffu, f.bad())) v = stencil_component<R>(own, other, t, fp64_sum, fp64_sum);
 					if (c) y.y = v;
 					else y.x = v;
 				}
@@ -257,7 +278,12 @@ StencilKernel stencil_kernel_of(bool team, bool win) {
 
 StencilKernel stencil_kernel(int radius, bool team, bool win) {
 	if (win && team) return nullptr;
-	return radius == 7 ? stencil_kernel_of<7>(team, win) : radius == 11 ? stencil_kernel_of<11>(team, win) : nullptr;
+	switch (radius) {
+		case 7: return stencil_kernel_of<7>(team, win);
+		case 11: return stencil_kernel_of<11>(team, win);
+		case 13: return stencil_kernel_of<13>(team, win);
+		default: return nullptr;
+	}
 }
 
 }  // namespace
@@ -268,7 +294,7 @@ const void *dnls_stencil_kernel_ptr(int radius, bool team, bool windowed) {
 
 size_t dnls_stencil_smem(uint32_t len, int lanes, int radius) {
 	const size_t chains = lanes > 32 ? 1 : size_t(4) * (32 / lanes);
-	const size_t consts = radius == 7 ? kStencilConsts<7> : kStencilConsts<11>;
+	const size_t consts = radius == 7 ? kStencilConsts<7> : radius == 11 ? kStencilConsts<11> : kStencilConsts<13>;
 	return (consts + chains * 2 * (len + 2 * size_t(radius))) * sizeof(double2);
 }
 

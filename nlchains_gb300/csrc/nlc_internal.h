@@ -243,9 +243,9 @@ struct DnlsArgs {
 };
 cudaError_t launch_dnls_move(const DnlsArgs &a, double2 *psi, int blocks, int threads, size_t smem,
                              int team_block, cudaStream_t stream);
-// DNLS with the linear sub-steps as a real-space stencil (nlc_dnls_stencil.cu) of radius R (instantiated: 7
-// and 11), the sites of a chain (or window) taken row by row by `lanes` threads
-constexpr int kMaxStencilRadius = 11;
+// DNLS with the linear sub-steps as a real-space stencil (nlc_dnls_stencil.cu) of radius R (instantiated: 7,
+// 11 and 13), the sites of a chain (or window) taken row by row by `lanes` threads
+constexpr int kMaxStencilRadius = 13;
 struct DnlsStencilArgs {
 	uint32_t n, copies, steps, seg;
 	int lanes;

@@ -725,14 +725,19 @@ static uint32_t dnls_window_steps(uint32_t win_len, int radius) {
 }
 
 // DNLS in the real-space stencil form (nlc_dnls_stencil.cu), where it applies: the propagator's taps
-// beyond radius 11 below 2^-64 (dt d_k up to ~0.05) and n >= 2R + 2; otherwise P.dnls_stencil stays false
+// beyond radius 13 below 2^-64 (dt up to ~0.15) and n >= 2R + 2; otherwise P.dnls_stencil stays false
 // and the plan takes the Fourier form.
 static int setup_dnls_stencil(nlc_plan &P) {
 	const uint32_t n = P.m.chain_length;
 	DnlsStencilArgs &a = P.sa;
 	const int need = dnls_stencil_coefficients(P.m.dt, kMaxStencilRadius, a.c0m1, &a.taps[0][0], a.phase);
-	const int R = need <= 7 ? 7 : need <= kMaxStencilRadius ? kMaxStencilRadius : 0;
+	const int R = need <= 7 ? 7 : need <= 11 ? 11 : need <= kMaxStencilRadius ? kMaxStencilRadius : 0;
 	if (!R || n < uint32_t(2 * R + 2)) return NLC_OK;
+	// Many 32- or 48-site chains at radius 13: their three cheap passes (radix 4 twice, then 2 or 3) take
+	// less than the 54-operation stencil (5 steps of 16384 chains of 32 sites: 1.68 against 2.08 ms, of
+	// 4096: 0.52 against 0.55, of 2048: 0.42 against 0.29; 48 sites, 2048 chains: 0.52 against 0.56; 64
+	// sites, 16384 chains: 3.56 against 3.33)
+	if (R == 13 && (n == 32 || n == 48) && uint64_t(P.m.copies) * n >= (3u << 15)) return NLC_OK;
 	int lanes = 0, sites = 0;
 	// NLC_DNLS_SITES=<E> restricts the shapes to E sites per lane (used by the tests to cover every
 	// instantiation); NLC_FORCE_WINDOW=<G> integrates in windows of G lanes where a block would hold

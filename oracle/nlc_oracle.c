@@ -512,18 +512,18 @@ int nlo_dnls_stencil_coefficients(double dt, int max_radius, double *c0m1, doubl
 	return radius;
 }
 
-#define NLO_STENCIL_MAX 11
+#define NLO_STENCIL_MAX 13
 
 typedef struct {
-	int radius;   /* the instantiated radius the engine runs: 7, or 11 */
+	int radius;   /* the instantiated radius the engine runs: 7, 11 or 13 */
 	double c0m1[7], taps[7 * NLO_STENCIL_MAX], phase[7];
 	double tab[2 * NLO_SINCOS_TABLE];
 } stencil_consts;
 
-/* 0 when the engine's stencil form does not apply to this dt (taps beyond radius 11) */
+/* 0 when the engine's stencil form does not apply to this dt (taps beyond radius 13) */
 static int make_stencil(double dt, stencil_consts *S) {
 	const int need = nlo_dnls_stencil_coefficients(dt, NLO_STENCIL_MAX, S->c0m1, S->taps, S->phase);
-	S->radius = need <= 7 ? 7 : need <= NLO_STENCIL_MAX ? NLO_STENCIL_MAX : 0;
+	S->radius = need <= 7 ? 7 : need <= 11 ? 11 : need <= NLO_STENCIL_MAX ? NLO_STENCIL_MAX : 0;
 	sincos_table_1024(S->tab);
 	return S->radius;
 }

@@ -70,10 +70,12 @@ def test_bits_at_edge_operands(gpu, monkeypatch, model, params, n, lanes):
     assert not bad.any(), f"rows {np.unique(np.nonzero(bad)[0])}: {np.count_nonzero(bad)} values differ"
 
 
-# sites per lane 1 .. 16 (rows over several chains of a warp, one chain of a warp, a block), both radii, and windows
+# sites per lane 1 .. 16 (rows over several chains of a warp, one chain of a warp, a block), every radius, and
+# windows
 @pytest.mark.parametrize("n,dt,sites,window", [(16, 0.01, 0, 0), (33, 0.01, 1, 0), (64, 0.01, 2, 0), (24, 0.05, 12, 0),
                                                (100, 0.05, 8, 0), (250, 0.01, 1, 0), (515, 0.01, 16, 0),
-                                               (1021, 0.05, 4, 0), (1300, 0.01, 0, 64), (2100, 0.05, 0, 96)])
+                                               (1021, 0.05, 4, 0), (1300, 0.01, 0, 64), (2100, 0.05, 0, 96),
+                                               (28, 0.1, 0, 0), (200, 0.15, 4, 0), (501, 0.1, 8, 0), (2100, 0.1, 0, 96)])
 def test_dnls_bits_at_edge_operands(gpu, monkeypatch, n, dt, sites, window):
     """The DNLS stencil form on the same states (phi + i pi as psi: real, imaginary and zero sites, angles on
     both sides of 2^-4 within a warp)."""
