@@ -20,11 +20,20 @@
 
 namespace nlc {
 
+// A mode's energy from the transform on the FP64 pipe, where the integer-pipe products do not hold
+// (nlc_intfp.cuh): |psi_k|^2, and |a_k Z_k + b_k conj Z_{n-k}|^2.
+__device__ __noinline__ double norm_fp64(double2 z) { return dfma(z.x, z.x, dmul(z.y, z.y)); }
+__device__ __noinline__ double mode_energy_fp64(double ak, double bk, double2 zk, double2 zm) {
+	const double re = dfma(ak, zk.x, dmul(bk, zm.x));
+	const double im = dfma(ak, zk.y, -dmul(bk, zm.y));
+	return dfma(re, re, dmul(im, im));
+}
+
 // One team (warp, or whole block when BLOCK) per chain; shared memory per team: 2 n complex
 // (ping-pong).  Each team accumulates its chains into its own row of `partials` (row = block *
 // teams + team), so no two threads ever add into the same element.
 template <bool BLOCK>
-__global__ void lin_fft_kernel(const double2 *__restrict__ state, const DiagArgs a) {
+__global__ void __launch_bounds__(BLOCK ? 512 : 128) lin_fft_kernel(const double2 *__restrict__ state, const DiagArgs a) {
 	extern __shared__ double2 sm[];
 	const int n = int(a.n);
 	const int T = BLOCK ? blockDim.x : 32;
@@ -38,25 +47,43 @@ __global__ void lin_fft_kernel(const double2 *__restrict__ state, const DiagArgs
 	for (int k = t; k < n; k += T) acc[k] = 0.;
 
 	const bool dnls = a.model == NLC_DNLS;
-	const FpOnes &k1 = a.fft.k1;
+	const FpOnes k1 = in_register(a.fft.k1, lane_zero(a.fft.k1));
 	for (unsigned long long chain = (unsigned long long) blockIdx.x * teams + team; chain < a.copies;
 	     chain += (unsigned long long) gridDim.x * teams) {
 		const double2 *src = state + chain * (unsigned long long) n;
 		for (int k = t; k < n; k += T) x[k] = src[k];
 		team_sync<BLOCK>();
-		const double2 *Z = fft_team<BLOCK, false>(a.fft, x, y, t, T);
+		const double2 *Z = fft_team<BLOCK, false>(a.fft, k1, x, y, t, T);
 		if (dnls) {
 			for (int k = t; k < n; k += T) {
 				const double2 z = Z[k];
-				acc[k] = fadd(acc[k], dfma(z.x, z.x, fmul(z.y, z.y, k1)), k1);
+				IntFlags f;
+				double e;
+				if (a.mixed) {
+					e = dfma(z.x, z.x, int_mul(z.y, z.y, f));
+					if (any_bad(f)) e = norm_fp64(z);
+				} else {
+					e = dfma(z.x, z.x, fmul(z.y, z.y, k1));
+				}
+				acc[k] = fadd(acc[k], e, k1);
 			}
 		} else {
 			for (int k = t; k < n; k += T) {
 				const double2 zk = Z[k], zm = Z[k ? n - k : 0];
 				const double ak = a.coef_a[k], bk = a.coef_b[k];
-				const double re = dfma(ak, zk.x, fmul(bk, zm.x, k1));
-				const double im = dfma(ak, zk.y, -fmul(bk, zm.y, k1));
-				acc[k] = fadd(acc[k], dfma(re, re, fmul(im, im, k1)), k1);
+				IntFlags f;
+				double e;
+				if (a.mixed) {
+					const double re = dfma(ak, zk.x, int_mul(bk, zm.x, f));
+					const double im = dfma(ak, zk.y, -int_mul(bk, zm.y, f));
+					e = dfma(re, re, int_mul(im, im, f));
+					if (any_bad(f)) e = mode_energy_fp64(ak, bk, zk, zm);
+				} else {
+					const double re = dfma(ak, zk.x, fmul(bk, zm.x, k1));
+					const double im = dfma(ak, zk.y, -fmul(bk, zm.y, k1));
+					e = dfma(re, re, fmul(im, im, k1));
+				}
+				acc[k] = fadd(acc[k], e, k1);
 			}
 		}
 		team_sync<BLOCK>();
@@ -68,7 +95,7 @@ __global__ void lin_fft_kernel(const double2 *__restrict__ state, const DiagArgs
 // formed in FP32; the sum over chains stays in the FP64 partial rows.  The error against the FP64
 // path is that of an FP32 transform, ~1e-7 of the largest mode energies.
 template <bool BLOCK>
-__global__ void lin_fft32_kernel(const double2 *__restrict__ state, const DiagArgs a) {
+__global__ void __launch_bounds__(BLOCK ? 512 : 128) lin_fft32_kernel(const double2 *__restrict__ state, const DiagArgs a) {
 	extern __shared__ float2 smf[];
 	const int n = int(a.n);
 	const int T = BLOCK ? blockDim.x : 32;
@@ -186,7 +213,7 @@ __device__ __forceinline__ double ic_uniform(unsigned long long key, unsigned lo
 }
 
 template <bool BLOCK>
-__global__ void ic_kernel(double2 *__restrict__ state, const DiagArgs a, const IcArgs c) {
+__global__ void __launch_bounds__(BLOCK ? 512 : 128) ic_kernel(double2 *__restrict__ state, const DiagArgs a, const IcArgs c) {
 	extern __shared__ double2 sm[];
 	const int n = int(a.n);
 	const int T = BLOCK ? blockDim.x : 32;
@@ -196,6 +223,7 @@ __global__ void ic_kernel(double2 *__restrict__ state, const DiagArgs a, const I
 	const int len = a.fft.len;
 	double2 *x = BLOCK && a.gscratch ? a.gscratch + (size_t) blockIdx.x * 2 * len : sm + (size_t) team * 2 * len;
 	double2 *y = x + len;
+	const FpOnes k1 = in_register(a.fft.k1, lane_zero(a.fft.k1));
 	for (unsigned long long chain = (unsigned long long) blockIdx.x * teams + team; chain < a.copies;
 	     chain += (unsigned long long) gridDim.x * teams) {
 		const unsigned long long copy = c.first_copy + chain;
@@ -245,7 +273,7 @@ __global__ void ic_kernel(double2 *__restrict__ state, const DiagArgs a, const I
 			w = y;
 		}
 		double2 *o = w == x ? y : x;
-		const double2 *r = fft_team<BLOCK, true>(a.fft, w, o, t, T);
+		const double2 *r = fft_team<BLOCK, true>(a.fft, k1, w, o, t, T);
 		const double inv_n = 1. / n;
 		for (int k = t; k < n; k += T) dst[k] = make_double2(r[k].x * inv_n, r[k].y * inv_n);
 		team_sync<BLOCK>();

@@ -45,6 +45,7 @@ __global__ void __launch_bounds__(BLOCK ? 512 : 128, BLOCK ? 2 : 8) dnls_move_ke
 	double2 *buf0 = BLOCK && a.gscratch ? a.gscratch + (size_t) blockIdx.x * 2 * len : sm + (size_t) team * 2 * len;
 	double2 *buf1 = buf0 + len;
 	const unsigned long long units = (a.copies + per_warp - 1) / per_warp;
+	const FpOnes k1 = in_register(a.fft.k1, lane_zero(a.fft.k1));
 
 	for (;;) {
 		// the next unit from the self-resetting counter: a chain (BLOCK) or a warp's chains
@@ -76,13 +77,13 @@ __global__ void __launch_bounds__(BLOCK ? 512 : 128, BLOCK ? 2 : 8) dnls_move_ke
 				// element (beyond n: the zero padding of the convolution form), the propagator (or
 				// the convolution kernel's spectrum) as its last pass writes each element
 				auto rotate = [&](int j, double2 v) {
-					return j < n ? nonlinear_rotate(v, -coef, a.sctab, a.sc, a.fft.k1) : make_double2(0., 0.);
+					return j < n ? nonlinear_rotate(v, -coef, a.sctab, a.sc, k1) : make_double2(0., 0.);
 				};
 				const double2 *tab = a.conv_tables ? a.conv_tables + (size_t) k * len : a.lin_tables + (size_t) k * n;
-				auto propagate = [&](int j, double2 v) { return cmul(v, tab[j], a.fft.k1); };
-				double2 *r = stockham_team<BLOCK, false>(a.fft, x, y, t, T, rotate, propagate);
+				auto propagate = [&](int j, double2 v) { return cmul(v, tab[j], k1); };
+				double2 *r = stockham_team<BLOCK, false>(a.fft, k1, x, y, t, T, rotate, propagate);
 				double2 *o = r == x ? y : x;
-				x = stockham_team<BLOCK, true>(a.fft, r, o, t, T);
+				x = stockham_team<BLOCK, true>(a.fft, k1, r, o, t, T);
 				y = x == buf0 ? buf1 : buf0;
 			}
 		}
@@ -90,7 +91,7 @@ __global__ void __launch_bounds__(BLOCK ? 512 : 128, BLOCK ? 2 : 8) dnls_move_ke
 			if (a.seg & NLC_SEG_OPEN)
 				for (int j = t; j < n; j += T) g[j] = x[j];
 			else
-				for (int j = t; j < n; j += T) g[j] = nonlinear_rotate(x[j], -a.nl_final, a.sctab, a.sc, a.fft.k1);
+				for (int j = t; j < n; j += T) g[j] = nonlinear_rotate(x[j], -a.nl_final, a.sctab, a.sc, k1);
 		}
 		team_sync<BLOCK>();
 	}

@@ -25,6 +25,7 @@
 
 #include "nlc_device.cuh"
 #include "nlc_internal.h"
+#include "nlc_intfp.cuh"
 
 namespace nlc {
 
@@ -51,10 +52,14 @@ __device__ __forceinline__ double2 twiddle(const double2 *__restrict__ tw, int e
 	const double2 w = tw[e];
 	return INV ? make_double2(w.x, -w.y) : w;
 }
-// multiply by -i (forward) or +i (inverse)
+// multiply by -i (forward) or +i (inverse); the sign is flipped as bits (a negation that does not fold
+// into an FMA's operand is an FP64 instruction)
+__device__ __forceinline__ double negate(double v) {
+	return __hiloint2double(__double2hiint(v) ^ int(0x80000000u), __double2loint(v));
+}
 template <bool INV>
 __device__ __forceinline__ double2 rot_mi(double2 a) {
-	return INV ? make_double2(-a.y, a.x) : make_double2(a.y, -a.x);
+	return INV ? make_double2(negate(a.y), a.x) : make_double2(a.y, negate(a.x));
 }
 
 // a (1 + i t) (forward) or a (1 - i t) (inverse): two FMAs
@@ -76,13 +81,13 @@ struct NoMap {
 
 // One Stockham pass r (radix P.radix[r], Ns points already combined) from x to y.  PRE / POST: the
 // pass applies `pre` to its inputs (the first pass) / `post` to its outputs (the last pass); they
-// are template flags so that the other passes carry no trace of the maps.
+// are template flags so that the other passes carry no trace of the maps.  k: the FP64 constants in
+// vector registers (nlc_device.cuh).
 template <bool BLOCK, bool INV, bool PRE, bool POST, class Pre, class Post>
-__device__ __forceinline__ void stockham_pass(const FftPlanDev &P, int r, int Ns, double2 *x, double2 *y, int t, int T,
-                                              const Pre &pre, const Post &post) {
+__device__ __forceinline__ void stockham_pass(const FftPlanDev &P, const FpOnes &k, int r, int Ns, double2 *x, double2 *y,
+                                              int t, int T, const Pre &pre, const Post &post) {
 	const int n = P.len;
 	const double2 *__restrict__ tw = P.tw;
-	const FpOnes &k = P.k1;
 	const int p = P.radix[r];
 	const int m = n / p;
 	const double2 *__restrict__ g = P.gw + P.gw_off[r];
@@ -119,9 +124,21 @@ __device__ __forceinline__ void stockham_pass(const FftPlanDev &P, int r, int Ns
 	if (p == 4) {
 		if (Ns == 1) {
 			for (int b = t; b < m; b += T) {
+				// sixteen additions: on the integer pipes, or on the FP64 pipe (P.fp64_first, or operands that
+				// ask for it)
 				const double2 a0 = in(b, 0), a1 = in(b, 1), a2 = in(b, 2), a3 = in(b, 3);
-				const double2 b0 = cadd(a0, a2, k), b1 = csub(a0, a2, k), b2 = cadd(a1, a3, k), b3 = rot_mi<INV>(csub(a1, a3, k));
-				store4(4 * b, b, cadd(b0, b2, k), cadd(b1, b3, k), csub(b0, b2, k), csub(b1, b3, k));
+				double2 X0, X1, X2, X3;
+				auto butterfly = [&](auto add, auto sub) {
+					const double2 b0 = add(a0, a2), b1 = sub(a0, a2), b2 = add(a1, a3), b3 = rot_mi<INV>(sub(a1, a3));
+					X0 = add(b0, b2), X1 = add(b1, b3), X2 = sub(b0, b2), X3 = sub(b1, b3);
+				};
+				IntFlags f;
+				if (!P.fp64_first)
+					butterfly([&](double2 u, double2 v) { return make_double2(int_add(u.x, v.x, f), int_add(u.y, v.y, f)); },
+					          [&](double2 u, double2 v) { return make_double2(int_sub(u.x, v.x, f), int_sub(u.y, v.y, f)); });
+				if (P.fp64_first || any_bad(f))
+					butterfly([&](double2 u, double2 v) { return cadd(u, v, k); }, [&](double2 u, double2 v) { return csub(u, v, k); });
+				store4(4 * b, b, X0, X1, X2, X3);
 			}
 		} else {
 			for (int b = t; b < m; b += T) {
@@ -249,16 +266,16 @@ __device__ __forceinline__ void stockham_pass(const FftPlanDev &P, int r, int Ns
 // Stockham transform of length P.len on x (shared memory), y the ping-pong buffer.  t / T: this
 // thread's index / size of the team.  Returns the buffer holding the result.
 template <bool BLOCK, bool INV, class Pre = NoMap, class Post = NoMap>
-__device__ double2 *stockham_team(const FftPlanDev &P, double2 *x, double2 *y, int t, int T, Pre pre = Pre(),
+__device__ double2 *stockham_team(const FftPlanDev &P, const FpOnes &k, double2 *x, double2 *y, int t, int T, Pre pre = Pre(),
                                   Post post = Post()) {
 	constexpr bool kPre = !std::is_same<Pre, NoMap>::value, kPost = !std::is_same<Post, NoMap>::value;
 	int Ns = 1;
 	for (int r = 0; r < P.nradix; r++) {
 		const bool first = r == 0, last = r == P.nradix - 1;
-		if (kPre && kPost && first && last) stockham_pass<BLOCK, INV, kPre, kPost>(P, r, Ns, x, y, t, T, pre, post);
-		else if (kPre && first) stockham_pass<BLOCK, INV, kPre, false>(P, r, Ns, x, y, t, T, pre, post);
-		else if (kPost && last) stockham_pass<BLOCK, INV, false, kPost>(P, r, Ns, x, y, t, T, pre, post);
-		else stockham_pass<BLOCK, INV, false, false>(P, r, Ns, x, y, t, T, pre, post);
+		if (kPre && kPost && first && last) stockham_pass<BLOCK, INV, kPre, kPost>(P, k, r, Ns, x, y, t, T, pre, post);
+		else if (kPre && first) stockham_pass<BLOCK, INV, kPre, false>(P, k, r, Ns, x, y, t, T, pre, post);
+		else if (kPost && last) stockham_pass<BLOCK, INV, false, kPost>(P, k, r, Ns, x, y, t, T, pre, post);
+		else stockham_pass<BLOCK, INV, false, false>(P, k, r, Ns, x, y, t, T, pre, post);
 		team_sync<BLOCK>();
 		double2 *sw = x;
 		x = y, y = sw;
@@ -346,10 +363,9 @@ __device__ __forceinline__ double2 conj2(double2 a) { return make_double2(a.x, -
 // convolution of smooth length m >= 2n - 1 by two Stockham passes; the backward transform uses the
 // conjugate chirp.  Returns the buffer holding X[0, n).
 template <bool BLOCK, bool INV>
-__device__ double2 *fft_team(const FftPlanDev &P, double2 *x, double2 *y, int t, int T) {
-	if (!P.bluestein) return stockham_team<BLOCK, INV>(P, x, y, t, T);
+__device__ double2 *fft_team(const FftPlanDev &P, const FpOnes &k, double2 *x, double2 *y, int t, int T) {
+	if (!P.bluestein) return stockham_team<BLOCK, INV>(P, k, x, y, t, T);
 	const int n = P.n, m = P.len;
-	const FpOnes &k = P.k1;
 	for (int j = t; j < m; j += T) {
 		if (j < n) {
 			const double2 w = P.chirp[j];
@@ -359,12 +375,12 @@ __device__ double2 *fft_team(const FftPlanDev &P, double2 *x, double2 *y, int t,
 		}
 	}
 	team_sync<BLOCK>();
-	double2 *r = stockham_team<BLOCK, false>(P, y, x, t, T);
+	double2 *r = stockham_team<BLOCK, false>(P, k, y, x, t, T);
 	double2 *o = r == y ? x : y;
 	const double2 *__restrict__ b = INV ? P.bi : P.bf;
 	for (int j = t; j < m; j += T) r[j] = cmul(r[j], b[j], k);
 	team_sync<BLOCK>();
-	double2 *c = stockham_team<BLOCK, true>(P, r, o, t, T);
+	double2 *c = stockham_team<BLOCK, true>(P, k, r, o, t, T);
 	for (int j = t; j < n; j += T) {
 		const double2 w = P.chirp[j];
 		c[j] = cmul(c[j], INV ? conj2(w) : w, k);

@@ -139,6 +139,10 @@ struct FftPlanDev {
 	const double2 *tw;     // tw[e] = exp(-2 pi i e / len), device
 	const double2 *gw;     // FMA-form twiddle entries of the radix-2/3/4 passes (fma_twiddle_entry), device
 	int gw_off[kMaxRadices];  // offset of pass r's entries in gw, in double2 units
+	// 1: the first pass's additions on the FP64 pipe: where zeros pad the inputs (the chirp-z transform
+	// and the convolution form: sums the integer pipes do not take), where the passes run from global
+	// memory, and where a scheduler has one warp or none (its integer and FP64 work do not overlap)
+	int fp64_first;
 	int bluestein;         // 1: chirp-z transform through a length-m cyclic convolution
 	const double2 *chirp;  // exp(-i pi j^2 / n), j < n
 	const double2 *bf;     // FFT_m(b) / m, b_j = exp(+i pi j^2 / n) wrapped (forward transforms)
@@ -159,6 +163,7 @@ struct DiagArgs {
 	const double *omega;     // DNLS omega_k, dDNKG omegas
 	const double *eigT;      // dDNKG: eigenvectors, row-major by site: eigT[s*n + k] = e_k[s]
 	double *partials;        // [blocks][n]
+	int mixed;               // 1: the mode energies' products on the integer pipes (several warps per scheduler)
 	double2 *gscratch;       // block teams whose buffers exceed shared memory: [blocks][2][len]
 	int proj_chunk;          // dDNKG: sites per shared-memory chunk of the projection
 	const float2 *tw32;      // FP32 diagnostics (NLC_FLAG_FP32_DIAGNOSTICS): twiddles in FP32; NULL: FP64

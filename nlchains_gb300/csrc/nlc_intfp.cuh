@@ -33,6 +33,13 @@ struct IntFlags {
 	__device__ __forceinline__ bool bad() const { return (dmax > 31u) | (exmax > 1976u) | (rmin <= 0); }
 };
 
+// Whether a lane that is here now has to redo its operations on the FP64 pipe.  The vote keeps the warp
+// together: a lane that branched off alone can run what follows apart from the others, every FP64
+// instruction of it twice.  Where the operations to redo are few (up to about eight), they belong in a
+// function that is not inlined: under a branch they become predicated instructions, which occupy the
+// pipe whether redone or not.
+__device__ __forceinline__ bool any_bad(const IntFlags &f) { return __any_sync(__activemask(), f.bad()); }
+
 __device__ __forceinline__ uint64_t mul_wide(uint32_t a, uint32_t b) {
 	uint64_t r;
 	asm("mul.wide.u32 %0, %1, %2;" : "=l"(r) : "r"(a), "r"(b));

@@ -502,6 +502,7 @@ int setup_fft(nlc_plan &P, FftPlanDev &f, bool convolution) {
 	f.nradix = int(T.radices.size());
 	for (size_t i = 0; i < T.radices.size(); i++) f.radix[i] = T.radices[i];
 	f.bluestein = T.bluestein;
+	f.fp64_first = T.bluestein || T.len > smem_fft_len(P);
 	double2 *d = nullptr;
 	int rc = P.upload(&d, reinterpret_cast<const double2 *>(T.tw.data()), T.len);
 	if (rc) return rc;
@@ -629,21 +630,34 @@ int setup_diagnostics(nlc_plan &P) {
 			if ((rc = P.upload(&d_om, P.omega_host.data(), n))) return rc;   // for nlc_initial_state
 			g.coef_a = d_a, g.coef_b = d_b, g.omega = d_om;
 		}
-		// a warp per chain up to a 1024-point pass (2 x 16 KiB ping-pong), else a 256-thread block
 		const uint32_t len = uint32_t(g.fft.len);
-		if (len <= 1024) {
+		const bool compact = P.m.flags & NLC_FLAG_COMPACT_DIAG;
+		if (len <= 256) {
+			// a warp per chain, four chains per block
 			P.diag_team_block = 0;
 			P.diag_threads = 128;
 			const int teams = 4;
 			P.diag_smem = size_t(teams) * 2 * len * sizeof(double2);
 			const unsigned long long groups = (P.m.copies + teams - 1) / teams;
-			P.diag_blocks = int(std::min<unsigned long long>(groups, (P.m.flags & NLC_FLAG_COMPACT_DIAG ? 1ull : 4ull) * sms));
+			P.diag_blocks = int(std::min<unsigned long long>(groups, (compact ? 1ull : 4ull) * sms));
 			P.diag_rows = P.diag_blocks * teams;
 		} else {
+			// A block per chain: the chain's two buffers in shared memory bound the chains per SM, so the
+			// threads per chain are what fills the schedulers (the fastest of 32 .. 512 at each length:
+			// 512-point passes 0.41 ms with 64 threads for 16384 chains, 0.54 with a warp each, four to a
+			// block; 1024-point passes 0.45 with 128 for 8192 chains against 0.80; 5000 points 0.57 with 512
+			// against 0.62 with 256), and more where there are fewer chains than fill the GPU (64 chains of
+			// 1024 points: 39 us with 256 threads, 55 with 64)
 			P.diag_team_block = 1;
-			P.diag_threads = 256;
+			int T = len <= 512 ? 64 : len <= 2048 ? 128 : len <= 3072 ? 256 : 512;
+			while (T < 512 && uint32_t(T) * 4 < len && (unsigned long long) P.m.copies * T < 256ull * sms) T <<= 1;
+			P.diag_threads = T;
 			P.diag_smem = size_t(2) * len * sizeof(double2);
-			P.diag_blocks = int(std::min<unsigned long long>(P.m.copies, (P.m.flags & NLC_FLAG_COMPACT_DIAG ? 1ull : 2ull) * sms));
+			// resident blocks, in shared memory and (at 125 registers) in the register file
+			int per_sm = int(std::min<size_t>(P.prop.sharedMemPerMultiprocessor / (P.diag_smem + 1024), size_t(512 / T)));
+			per_sm = std::max(per_sm, 2);
+			if (compact) per_sm = len <= 1024 ? 2 : 1;
+			P.diag_blocks = int(std::min<unsigned long long>(P.m.copies, (unsigned long long) per_sm * sms));
 			P.diag_rows = P.diag_blocks;
 			if (len > smem_fft_len(P)) {
 				// the two buffers of each block in global memory (L2-resident at these sizes)
@@ -652,6 +666,8 @@ int setup_diagnostics(nlc_plan &P) {
 				if ((rc = P.dalloc(&g.gscratch, size_t(P.diag_blocks) * 2 * len))) return rc;
 			}
 		}
+		g.mixed = (unsigned long long) P.diag_rows * (P.diag_team_block ? P.diag_threads / 32 : 1) >= 8ull * sms;
+		if (!g.mixed) g.fft.fp64_first = 1;
 		// FP32 diagnostics: for direct transforms held in shared memory (padded lengths and
 		// global-memory passes keep the FP64 transform)
 		if ((P.m.flags & NLC_FLAG_FP32_DIAGNOSTICS) && !g.fft.bluestein && !g.gscratch) {
