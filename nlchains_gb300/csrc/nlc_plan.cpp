@@ -189,13 +189,13 @@ int validate(const nlc_model *m) {
 	return NLC_OK;
 }
 
-// Candidate (G, E) for a chain of n sites: G power of two, E = ceil(n / G) in [2, 16] (E = 1 is not
-// instantiated), every lane holding E or E - 1 >= 1 sites.
+// Candidate (G, E) for a chain of n sites: G power of two, E = ceil(n / G) in [1, 16], every lane
+// holding E or E - 1 >= 1 sites (E = 1: n = G).
 std::vector<std::pair<int, int>> shape_candidates(uint32_t n) {
 	std::vector<std::pair<int, int>> c;
 	for (int G = 1; G <= kMaxLanesPerChain; G <<= 1) {
 		const uint32_t E = (n + G - 1) / G;
-		if (E < 2 || E > uint32_t(kMaxSitesPerLane)) continue;
+		if (E > uint32_t(kMaxSitesPerLane) || uint64_t(G) * (E - 1) >= n || uint32_t(G) > n) continue;
 		c.emplace_back(G, int(E));
 	}
 	return c;

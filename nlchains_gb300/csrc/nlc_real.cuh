@@ -4,7 +4,7 @@
 // DNKG_FPUT_Toda.cu:82-259, dDNKG.cu:25-196) with one kernel family:
 //
 // * a chain of n sites is spread over G lanes (G a power of two, 1 .. 1024), each lane holding E or
-//   E - 1 consecutive sites in registers (E a compile-time constant 2..16, so arrays index
+//   E - 1 consecutive sites in registers (E a compile-time constant 1..16, so arrays index
 //   statically), the first n - G(E - 1) lanes holding E -- the reference's warp layout
 //   (DNKG_FPUT_Toda.cu:94-106) generalised to any group width;
 // * groups of G <= 32 lanes exchange halos with width-G shuffles; for G > 32 one block holds one
@@ -157,11 +157,13 @@ __device__ __forceinline__ void sub_batch(double *out, const double *a, const do
 
 template <int MODEL, int E, int VAR, bool WIN>
 __global__ void real_move_kernel_t(double2 *__restrict__ state, const RealArgs a) {
-	// Additions (and DNKG's squares) on the integer pipes beside the FP64 ones, from 4 sites per lane
-	// on.  Shapes of 2 or 3 sites per lane are those of ensembles too small to give a scheduler more
-	// than one or two warps: there the two pipes do not overlap (a warp issues in order), and an
-	// operation costs 75 clocks against 64.
-	constexpr bool INT = E >= 4;
+	// Operations on the integer pipes from 4 sites per lane on, and for Toda (12 operations a site) always.
+	// Lanes of fewer sites are those of ensembles too small to fill the schedulers, or of short chains:
+	// with a warp or two per scheduler the two pipes hardly overlap (a warp issues in order) and an
+	// operation costs 75 clocks against 64 (FPUT N = 64, 100 steps, one site per lane: 232 us for 96 chains
+	// with the FP64 pipe alone, 403 with both; 1024 chains 497 against 679; Toda N = 128, 512 chains
+	// 1082 against 958).
+	constexpr bool INT = E >= 4 || MODEL == NLC_TODA;
 	__shared__ double xbuf[4 * 32];
 	__shared__ double s_tab[MODEL == NLC_TODA ? kExpTable : 1];
 	__shared__ unsigned long long s_unit;
@@ -270,7 +272,7 @@ __global__ void real_move_kernel_t(double2 *__restrict__ state, const RealArgs a
 			} else {
 				x[j + 1] = 0., p[j] = 0.;
 			}
-			if constexpr (INT && MODEL == NLC_DDNKG && VAR)
+			if constexpr (MODEL == NLC_DDNKG && VAR)
 				mv_bad |= uint32_t(__double2hiint(mv[j])) - 0x04000000u > 0x78000000u;
 		}
 
@@ -430,12 +432,13 @@ struct RealKernels {
 		return variant ? real_move_kernel_t<MODEL, E, 1, WIN> : real_move_kernel_t<MODEL, E, 0, WIN>;
 	}
 	// Two halves of about equal compile time, so that a model whose kernels take long to compile can
-	// build them in two translation units: lanes of 2..13 sites and 4-site windows; lanes of 14..16
+	// build them in two translation units: lanes of up to 13 sites and 4-site windows; lanes of 14..16
 	// sites and the wider windows
 	static bool is_short(int e, bool win) { return win ? e == 4 : e <= 13; }
 	static K lookup_short(int variant, int e, bool win) {
 		if (win) return e == 4 ? get<4, true>(variant) : nullptr;
 		switch (e) {
+			case 1: return get<1>(variant);
 			case 2: return get<2>(variant);
 			case 3: return get<3>(variant);
 			case 4: return get<4>(variant);

@@ -1,4 +1,4 @@
-// Toda's resident-integrator instantiations for lanes of 2..13 sites and 4-site windows (the rest in
+// Toda's resident-integrator instantiations for lanes of up to 13 sites and 4-site windows (the rest in
 // nlc_real_toda.cu).
 #include "nlc_real.cuh"
 
