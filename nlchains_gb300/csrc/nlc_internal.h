@@ -329,6 +329,7 @@ struct EnergyArgs {
 	int model;
 	uint32_t n, copies;
 	double m, alpha, beta;
+	double toda_scale;        // 1 / (4 alpha^2)
 	const double *mp2_site;   // dDNKG: m_s + 2 (device)
 };
 cudaError_t launch_energies(const EnergyArgs &a, const double2 *state, double *out, cudaStream_t stream);

@@ -1372,6 +1372,7 @@ extern "C" int nlc_energies(nlc_plan *P, const void *state, double *energies, vo
 	e.model = P->m.model;
 	e.n = P->m.chain_length, e.copies = P->m.copies;
 	e.m = P->m.m, e.alpha = P->m.alpha, e.beta = P->m.beta;
+	if (e.model == NLC_TODA) e.toda_scale = 1 / (4 * e.alpha * e.alpha);
 	e.mp2_site = P->ra.mp2_site;
 	return cuda_status(launch_energies(e, static_cast<const double2 *>(state), energies, static_cast<cudaStream_t>(stream)),
 	                   "energies launch");

@@ -38,9 +38,9 @@ def edge_states(n, seed):
     return np.array(rows)
 
 
-# lanes x sites per lane: one warp with full lanes and short ones, up to and beyond a batch of 8, several
+# one site per lane, in a warp and in a block, two; then from four on: one warp with full lanes and short ones, up to and beyond a batch of 8, several
 # chains per warp, a block
-SHAPES = [(4, 1), (8, 1), (9, 1), (16, 1), (61, 8), (64, 8), (128, 16), (100, 8), (500, 32), (512, 64), (1000, 128)]
+SHAPES = [(16, 16), (64, 64), (256, 256), (5, 4), (200, 128), (4, 1), (8, 1), (9, 1), (16, 1), (61, 8), (64, 8), (128, 16), (100, 8), (500, 32), (512, 64), (1000, 128)]
 MODELS = [("DNKG", dict(m=1.0, beta=1.0)), ("DNKG", dict(m=0.0, beta=1.0)), ("DNKG", dict(m=-2.5, beta=1.0)), ("DNKG", dict(m=-2.0, beta=1.0)),
           ("DNKG", dict(m=0.3, beta=0.7)), ("dDNKG", dict(beta=1.0)), ("FPUT", dict(alpha=0.0, beta=1.0)),
           ("FPUT", dict(alpha=0.25, beta=0.5)), ("Toda", dict(alpha=0.5)), ("Toda", dict(alpha=0.75))]
