@@ -469,22 +469,37 @@ double block_step_ops(int model, uint32_t n, uint32_t len, bool bluestein, int c
 	return per_site * double(n) * chains_per_block / eff;
 }
 
-// Windowed tier: the launchable block shape (G > 32 lanes of E sites, one window per block) with
-// the most sites G E.  Longer windows waste less on their discarded ends.
-RealShape window_shape(const nlc_plan &P, int model, int variant, int only_lanes) {
+// Estimated clocks of a step of `units` blocks of G > 32 lanes of E sites (a chain or a window each).  A row
+// of a block (one site of each lane) takes an SM about 350 clocks with a few warps (latency) and 51 a
+// warp with many (DNKG; the other models rank alike).
+double block_tier_cost(const nlc_plan &P, int model, int variant, const RealShape &s, bool win, double units) {
+	int per_sm = 1;
+	cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, real_move_kernel(model, variant, s.sites, win), s.threads, 0);
+	const double warps = units * (s.lanes / 32) / P.prop.multiProcessorCount, resident = std::max(per_sm, 1) * (s.lanes / 32);
+	const double row = std::max(350., 51. * std::min(warps, resident)) * std::max(1., warps / resident);
+	return 7 * s.sites * row * (per_sm < 2 ? 1.3 : 1.);   // nothing hides the barriers of a lone block
+}
+
+// Windowed tier: the block shape (G > 32 lanes of E sites, one window per block) of the least estimated
+// time per step, a launch of s steps costing about 8000 clocks more, and the state's way through memory.
+// DNKG n = 20000, 96 chains, 50 steps: 4.49 ms in windows of 64 x 16 sites, 4.66 in 128 x 16, 6.54 in
+// 512 x 8; one chain 0.61 ms in 256 x 4, 1.14 in 64 x 16.
+RealShape window_shape(const nlc_plan &P, int model, int variant, int only_lanes, double *cost_out = nullptr) {
 	RealShape best{};
-	for (int G = kMaxLanesPerChain; G > 32; G >>= 1)
+	double least = 0;
+	for (int G = 64; G <= kMaxLanesPerChain; G <<= 1)
 		for (int E = kMaxSitesPerLane; E >= 2; E--) {
 			if (only_lanes && G != only_lanes) break;
-			if (uint64_t(G) * E <= uint64_t(best.lanes) * best.sites) break;
-			if (uint64_t(G) * E >= P.m.chain_length) continue;
-			RealShape s{};
-			s.lanes = G, s.sites = E;
-			if (finish_shape(P, model, variant, s, G, true)) {
-				best = s;
-				break;
-			}
+			const uint32_t n = P.m.chain_length, len = uint32_t(G) * E, s = std::max<uint32_t>(1, len / 140), halo = 7 * s;
+			if (len >= n || 2 * halo >= len) continue;
+			RealShape sh{};
+			sh.lanes = G, sh.sites = E;
+			if (!finish_shape(P, model, variant, sh, G, true)) continue;
+			const double windows = double(P.m.copies) * ((n + len - 2 * halo - 1) / (len - 2 * halo));
+			const double cost = block_tier_cost(P, model, variant, sh, true, windows) + (8000. + 0.0102 * P.m.copies * n) / s;
+			if (only_lanes ? E > best.sites : !best.blocks || cost < least) least = cost, best = sh;
 		}
+	if (cost_out) *cost_out = least;
 	return best;
 }
 
@@ -1052,9 +1067,17 @@ extern "C" int nlc_plan_create(const nlc_model *model, nlc_plan **out) {
 		// (used by the tests to cover the windowed tier on short chains)
 		const char *force_win = std::getenv("NLC_FORCE_WINDOW");
 		if (force_win) P->rs = RealShape{};
+		// Chains on one block of 256 lanes or more also run in windows where those are estimated faster (few
+		// chains, or blocks too large to run two to an SM: DNKG n = 7000, 200 chains, 50 steps 4.88 ms on
+		// 512 lanes of 14 sites, 3.97 in windows; 16 chains of 4096 sites 1.59 and 0.6)
+		else if (P->rs.lanes >= 256 && !std::getenv("NLC_FORCE_LANES") && !(model->flags & NLC_FLAG_CANONICAL_SHAPE)) {
+			double cost = 0;
+			const RealShape w = window_shape(*P, mdl, P->variant, 0, &cost);
+			if (w.blocks && cost < 0.95 * block_tier_cost(*P, mdl, P->variant, P->rs, false, model->copies)) P->rs = RealShape{};
+		}
 		if (!P->rs.blocks) {
-			// longer than one block's registers hold: windows of the chain, ping-ponging between the
-			// caller's buffer and a second one of the same size
+			// longer than one block's registers hold, or faster so: windows of the chain, ping-ponging
+			// between the caller's buffer and a second one of the same size
 			P->rs = window_shape(*P, mdl, P->variant, force_win ? std::atoi(force_win) : 0);
 			if (!P->rs.blocks) return set_error(NLC_EUNSUPPORTED, "no launchable integrator shape for this chain_length");
 			P->win_len = uint32_t(P->rs.lanes) * P->rs.sites;

@@ -99,3 +99,36 @@ def test_dnls_bits_at_edge_operands(gpu, monkeypatch, n, dt, sites, window):
     assert np.isfinite(exp).all()
     bad = out.view(np.uint64) != exp.view(np.uint64)
     assert not bad.any(), f"rows {np.unique(np.nonzero(bad)[0])}: {np.count_nonzero(bad)} values differ"
+
+
+@pytest.mark.parametrize("model,params", [("DNKG", dict(m=1.0, beta=1.0)), ("DNKG", dict(m=0.3, beta=0.7)),
+                                          ("dDNKG", dict(beta=1.0)), ("FPUT", dict(alpha=0.25, beta=0.5)),
+                                          ("Toda", dict(alpha=0.5))], ids=lambda v: v if isinstance(v, str) else "")
+@pytest.mark.parametrize("n,lanes", [(2049, 256), (2500, 512), (3600, 256)])
+def test_chains_moved_to_windows_equal_one_block(gpu, monkeypatch, model, params, n, lanes):
+    """Lengths that a block would hold but that run in windows for few chains: the same bits as on a block,
+    over an odd and an even number of launches, in one batch and in several."""
+    if model == "dDNKG":
+        n, lanes = n // 4, 64
+        monkeypatch.setenv("NLC_FORCE_WINDOW", "64")
+    masses = ic.masses_uniform(n, seed=n) if model == "dDNKG" else None
+    r = np.random.RandomState(n)
+    state = 0.3 * r.standard_normal((3, n, 2))
+    state[1, ::3] = 0.0
+
+    def advance(batching, steps):
+        ctx = gpu.Context(0)
+        job = ctx.job(gpu.Model(model, n, 3, 0.05, masses=masses, **params), batching)
+        job.upload(state)
+        job.advance(steps)
+        out = job.download()
+        job.close()
+        ctx.close()
+        return out
+
+    assert gpu.Plan(gpu.Model(model, n, 3, 0.05, masses=masses, **params)).shape()["tier"] == 4
+    windows = [advance(b, 24) for b in (24, 8, 3)]
+    monkeypatch.delenv("NLC_FORCE_WINDOW", raising=False)
+    monkeypatch.setenv("NLC_FORCE_LANES", str(lanes))
+    for b, w in zip((24, 8, 3), windows):
+        assert np.array_equal(w.view(np.uint64), advance(b, 24).view(np.uint64)), b
