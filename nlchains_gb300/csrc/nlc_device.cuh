@@ -43,7 +43,7 @@ __device__ __forceinline__ FpOnes in_register(const FpOnes &k, int zero) {
 	return r;
 }
 __device__ __forceinline__ ExpConsts in_register(const ExpConsts &c, int zero) {
-	ExpConsts r;
+	ExpConsts r = c;
 	r.shifter = in_register(c.shifter, zero), r.inv_l = in_register(c.inv_l, zero);
 	r.l1 = in_register(c.l1, zero), r.l2 = in_register(c.l2, zero);
 	r.c3 = in_register(c.c3, zero), r.c2 = in_register(c.c2, zero);

@@ -25,6 +25,7 @@ struct ExpConsts {
 	double l1 = 0x1.62e42fefa39efp-12;             // ln 2 / 2048, leading part
 	double l2 = 0x1.abc9e3b39803fp-67;             // ln 2 / 2048, trailing part
 	double c3 = 1. / 6, c2 = 0.5;                  // Taylor coefficients of exp(r) - 1 - r (r^4/24 < 2^-54)
+	uint32_t inv1 = 0x171547u, inv0 = 0x652b82feu; // significand of inv_l = 1.44... x 2^11, high and low words
 };
 
 // Constants of the table-driven sincos (nlc_device.cuh sincos_table): Cody-Waite reduction by

@@ -159,13 +159,31 @@ __device__ __forceinline__ double int_to_double(int n) {
 	return __hiloint2double(int(n ? h | (b & 0x80000000u) : 0u), int(b << 29));
 }
 
-// exp_scaled (nlc_device.cuh) with the table index's value and the product of the polynomial on the
-// integer pipes: 6 of its 8 operations stay on the FP64 pipe.  Flagged where exp_scaled leaves its fast
-// path, and somewhat before.
+// The nearest integer to x inv_l, |x| < 4096 (the caller's flag), as the FP64 pipe's x inv_l + 1.5 2^52
+// rounds it: from the top 64 bits of the exact product's 106, flagged where the bits below the half
+// are all zeros (a tie) or all ones (what was cut off could carry).
+__device__ __forceinline__ int int_exp_index(double x, const ExpConsts &c, IntFlags &f) {
+	const uint32_t xh = __double2hiint(x), x0 = __double2loint(x), x1 = (xh & 0xfffffu) | 0x100000u;
+	const uint64_t mid = mad_wide(x0, c.inv1, mad_wide(x1, c.inv0, uint64_t(hi32(mul_wide(x0, c.inv0)))));
+	const uint64_t top = mad_wide(x1, c.inv1, uint64_t(hi32(mid)));
+	const uint64_t p = uint64_t(__funnelshift_l(lo32(mid), lo32(top), 22)) |
+	                   uint64_t(__funnelshift_l(lo32(top), hi32(top), 22)) << 32;   // the product's bits from 42 on
+	const int s = 1073 - int((xh >> 20) & 0x7ffu);   // the half's place in p
+	uint64_t twice, below;
+	asm("shr.u64 %0, %1, %2;" : "=l"(twice) : "l"(p), "r"(s));        // shifts of 64 and more give 0
+	asm("shl.b64 %0, %1, %2;" : "=l"(below) : "l"(p), "r"(64 - s));
+	f.rmin = min(f.rmin, s > 63 ? 1 : int((hi32(below) + 1u) >> 1));
+	const int n = int((lo32(twice) + 1u) >> 1), neg = int(xh) >> 31;
+	return (n ^ neg) - neg;
+}
+
+// exp_scaled (nlc_device.cuh) with the table's index, its value as a double and the product of the
+// polynomial on the integer pipes: 5 of its 8 operations stay on the FP64 pipe.  Flagged where exp_scaled
+// leaves its fast path, and somewhat before.
 __device__ __forceinline__ double exp_scaled_mixed(double x, const double *__restrict__ table, const FpOnes &k1,
                                                    const ExpConsts &c, IntFlags &f) {
 	f.rmin = min(f.rmin, 0x40b00000 - (__double2hiint(x) & 0x7fffffff));   // |x| < 4096: |n| < 2^24
-	const int n = __double2loint(dfma(x, c.inv_l, c.shifter));
+	const int n = int_exp_index(x, c, f);
 	const double nf = int_to_double(n);
 	double r = dfma(-nf, c.l1, x);
 	r = dfma(-nf, c.l2, r);

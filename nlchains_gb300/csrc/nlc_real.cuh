@@ -155,8 +155,16 @@ __device__ __forceinline__ void sub_batch(double *out, const double *a, const do
 	}
 }
 
+// Threads that a block may have, which caps the registers: at 512 (128 registers) four blocks of 128
+// threads share an SM, where the compiler's own choice of 130 to 138 leaves three (FPUT N = 459, 3001
+// chains, 50 steps: 4.82 -> 4.56 ms); more registers where 128 would spill.
+template <int MODEL, int E, bool WIN>
+constexpr int kMaxThreads = MODEL == NLC_DNKG    ? (WIN && E >= 12 ? 384 : 512)
+                            : MODEL == NLC_DDNKG ? (E <= 8 ? 512 : E <= 11 ? 384 : 256)
+                                                 : (E <= (WIN ? 11 : 12) ? 512 : 384);
+
 template <int MODEL, int E, int VAR, bool WIN>
-__global__ void real_move_kernel_t(double2 *__restrict__ state, const RealArgs a) {
+__global__ void __launch_bounds__(kMaxThreads<MODEL, E, WIN>) real_move_kernel_t(double2 *__restrict__ state, const RealArgs a) {
 	// Operations on the integer pipes from 4 sites per lane on, and for Toda (12 operations a site) always.
 	// Lanes of fewer sites are those of ensembles too small to fill the schedulers, or of short chains:
 	// with a warp or two per scheduler the two pipes hardly overlap (a warp issues in order) and an
