@@ -177,9 +177,38 @@ __device__ __forceinline__ int int_exp_index(double x, const ExpConsts &c, IntFl
 	return (n ^ neg) - neg;
 }
 
-// exp_scaled (nlc_device.cuh) with the table's index, its value as a double and the product of the
-// polynomial on the integer pipes: 5 of its 8 operations stay on the FP64 pipe.  Flagged where exp_scaled
-// leaves its fast path, and somewhat before.
+// 1 + a b, |a b| < 1/4 (flagged): the exact product's top 64 bits shifted to the scale of 2^-62, the rest
+// ORed into the lowest one, added to or subtracted from 2^62; the sum's leading bit is at 62 or 61.
+__device__ __forceinline__ double int_one_plus(double a, double b, IntFlags &f) {
+	const uint32_t ah = __double2hiint(a), a0 = __double2loint(a), bh = __double2hiint(b), b0 = __double2loint(b);
+	const uint32_t a1 = (ah & 0xfffffu) | 0x100000u, b1 = (bh & 0xfffffu) | 0x100000u;
+	const uint64_t low = mul_wide(a0, b0);
+	const uint64_t mid = mad_wide(a0, b1, mad_wide(a1, b0, uint64_t(hi32(low))));
+	const uint64_t top = mad_wide(a1, b1, uint64_t(hi32(mid)));
+	const uint64_t p = uint64_t(__funnelshift_l(lo32(mid), lo32(top), 22)) |
+	                   uint64_t(__funnelshift_l(lo32(top), hi32(top), 22)) << 32;   // the product's bits from 42 on
+	const int t = 2046 - int((ah >> 20) & 0x7ffu) - int((bh >> 20) & 0x7ffu);
+	uint64_t aligned, lost;
+	asm("shr.u64 %0, %1, %2;" : "=l"(aligned) : "l"(p), "r"(t));   // shifts of 64 and more give 0
+	asm("shl.b64 %0, %1, %2;" : "=l"(lost) : "l"(p), "r"(64 - t));
+	const uint32_t sticky = min(lo32(lost) | hi32(lost) | (lo32(mid) << 22) | lo32(low), 1u);
+	const uint32_t neg = uint32_t(int32_t(ah ^ bh) >> 31);
+	uint32_t rl, rh;
+	asm("{add.cc.u32 %0, %2, %3; addc.u32 %1, %4, 0x40000000;}"
+	    : "=r"(rl), "=r"(rh)
+	    : "r"((lo32(aligned) | sticky) ^ neg), "r"(0u - neg), "r"(hi32(aligned) ^ neg));
+	const uint32_t z = ~rh >> 30 & 1u;   // 1: below 1
+	const uint32_t drop = 10u - z, half = ((rl >> drop) & 1u) + (0x200u >> z) - 1u;
+	uint32_t ol, oh;
+	asm("{add.cc.u32 %0, %2, %3; addc.u32 %1, %4, 0;}" : "=r"(ol), "=r"(oh) : "r"(rl), "r"(half), "r"(rh));
+	f.rmin = min(f.rmin, t - 1);
+	return __hiloint2double(int((oh >> drop) + 0x3fe00000u - z * 0x100000u), int(__funnelshift_r(ol, oh, drop)));
+}
+
+// exp_scaled (nlc_device.cuh) with the table's index, its value as a double, the polynomial's last product
+// and (HALF) the sum before it on the integer pipes: 5 or 4 of its 8 operations stay on the FP64 pipe.
+// Flagged where exp_scaled leaves its fast path, and somewhat before.
+template <bool HALF>
 __device__ __forceinline__ double exp_scaled_mixed(double x, const double *__restrict__ table, const FpOnes &k1,
                                                    const ExpConsts &c, IntFlags &f) {
 	f.rmin = min(f.rmin, 0x40b00000 - (__double2hiint(x) & 0x7fffffff));   // |x| < 4096: |n| < 2^24
@@ -187,8 +216,7 @@ __device__ __forceinline__ double exp_scaled_mixed(double x, const double *__res
 	const double nf = int_to_double(n);
 	double r = dfma(-nf, c.l1, x);
 	r = dfma(-nf, c.l2, r);
-	double q = dfma(r, c.c3, c.c2);
-	q = dfma(q, r, k1.one);
+	const double h = dfma(r, c.c3, c.c2), q = HALF ? int_one_plus(h, r, f) : dfma(h, r, k1.one);
 	const double tj = table[n & (kExpTable - 1)];
 	const double v = dfma(tj, int_mul(q, r, f), tj);
 	const int k = n >> 11, hi = __double2hiint(v);

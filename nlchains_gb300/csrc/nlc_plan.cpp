@@ -1090,6 +1090,7 @@ extern "C" int nlc_plan_create(const nlc_model *model, nlc_plan **out) {
 			P->rs.blocks = int(std::min<unsigned long long>((model->copies + gpb - 1) / gpb, 0x7fffffffull));
 		}
 		a.lanes = P->rs.lanes;
+		a.mixed = (unsigned long long) model->copies * P->rs.lanes >= 64ull * P->prop.multiProcessorCount;
 		P->tier = P->win_len ? 4 : P->rs.lanes > 32 ? 2 : 1;
 		int per_sm = 1;
 		cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, real_move_kernel(mdl, P->variant, P->rs.sites, P->win_len != 0),

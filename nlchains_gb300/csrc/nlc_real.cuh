@@ -25,13 +25,15 @@
 //
 // Operations per site and sub-step, and where they run (the FP64 pipe is the bound; the integer
 // pipes work beside it):
-//   DNKG / dDNKG 6 (5 with beta == 1): the subtraction and, with beta == 1, the square plus m + 2 on
-//     the integer pipes, 4 (3) left on the FP64 pipe.  DNKG N = 128, 65536 chains, 100 steps: 53.8
-//     ms with all five on the FP64 pipe, 39.8 with the subtraction moved, 32.1 with the square too
-//     (26.1 G site-steps/s; the FP64 pipe 87% busy at the three operations it keeps).
-//   FPUT 7 (6 with alpha == 0 and beta == 1), Toda 13 (12 with 2 alpha == 1) including the 8-operation
-//     table exp: the two subtractions on the integer pipes.  FPUT N = 459, 3001 chains, 50 steps: 7.05
-//     -> 5.54 ms; Toda N = 128, 16384 chains, 100 steps: 32.9 -> 28.5 ms.
+//   DNKG / dDNKG 6 (5 with beta == 1): the subtraction and the square plus m + 2 (beta == 1) or beta x on
+//     the integer pipes, 3 (4) left on the FP64 pipe.  DNKG N = 128, 65536 chains, 100 steps: 53.8 ms with
+//     all five on the FP64 pipe, 39.8 with the subtraction moved, 32.1 with the square too, 29.7 with
+//     vector-register operands (28.2 G site-steps/s; the FP64 pipe 94% busy).
+//   FPUT 7 (6 with alpha == 0 and beta == 1): the two subtractions and the product d w, 4 (3) left.
+//     N = 459, 3001 chains, 50 steps with alpha: 7.05 -> 4.55 ms.
+//   Toda 13 (12 with 2 alpha == 1) including the 8-operation table exp: the two subtractions, the index,
+//     its value and half the polynomial of the exp, 6 left.  N = 128, 16384 chains, 100 steps: 32.9 ->
+//     17.2 ms (20.1 with the index and the polynomial's sum still on the FP64 pipe).
 #pragma once
 
 #include <type_traits>
@@ -119,14 +121,14 @@ __device__ __forceinline__ double bond_force(double d, const ForceConsts &c, con
 	}
 }
 // the same with its products on the integer pipes
-template <int MODEL, int VAR>
+template <int MODEL, int VAR, bool HALF>
 __device__ __forceinline__ double bond_force_mixed(double d, const ForceConsts &c, const FpOnes &k1, const double *tab,
                                                    IntFlags &f) {
 	if constexpr (MODEL == NLC_FPUT) {
 		const double h = VAR ? d : dfma(c.beta, d, c.alpha);
 		return int_mul(d, dfma(h, d, k1.one), f);
 	} else {
-		return exp_scaled_mixed(VAR ? d : int_mul(c.alpha2, d, f), tab, k1, c.ek, f);
+		return exp_scaled_mixed<HALF>(VAR ? d : int_mul(c.alpha2, d, f), tab, k1, c.ek, f);
 	}
 }
 
@@ -165,13 +167,6 @@ constexpr int kMaxThreads = MODEL == NLC_DNKG    ? (WIN && E >= 12 ? 384 : 512)
 
 template <int MODEL, int E, int VAR, bool WIN>
 __global__ void __launch_bounds__(kMaxThreads<MODEL, E, WIN>) real_move_kernel_t(double2 *__restrict__ state, const RealArgs a) {
-	// Operations on the integer pipes from 4 sites per lane on, and for Toda (12 operations a site) always.
-	// Lanes of fewer sites are those of ensembles too small to fill the schedulers, or of short chains:
-	// with a warp or two per scheduler the two pipes hardly overlap (a warp issues in order) and an
-	// operation costs 75 clocks against 64 (FPUT N = 64, 100 steps, one site per lane: 232 us for 96 chains
-	// with the FP64 pipe alone, 403 with both; 1024 chains 497 against 679; Toda N = 128, 512 chains
-	// 1082 against 958).
-	constexpr bool INT = E >= 4 || MODEL == NLC_TODA;
 	__shared__ double xbuf[4 * 32];
 	__shared__ double s_tab[MODEL == NLC_TODA ? kExpTable : 1];
 	__shared__ unsigned long long s_unit;
@@ -286,8 +281,8 @@ __global__ void __launch_bounds__(kMaxThreads<MODEL, E, WIN>) real_move_kernel_t
 
 		(void) mv_bad;
 		const double cd_lead = (seg & NLC_SEG_CONTINUE) ? a.cd0_merged : a.cd[0];
-		auto integrate = [&](auto shfl_tag) {
-		constexpr bool SHFL = decltype(shfl_tag)::value;
+		auto integrate = [&](auto shfl_tag, auto int_tag) {
+		constexpr bool SHFL = decltype(shfl_tag)::value, INT = decltype(int_tag)::value;
 		uint32_t rpos = 0;   // steps of the current round done (fused rounds, a.round_steps)
 		for (uint32_t i = 0; i < steps; i++) {
 			// a round boundary inside the launch: the closing drift of the round just done, then the
@@ -374,7 +369,7 @@ __global__ void __launch_bounds__(kMaxThreads<MODEL, E, WIN>) real_move_kernel_t
 #pragma unroll
 							for (int j = j0; j <= E && j < j0 + kIntBatch; j++) {
 								IntFlags &fj = j == E ? fe : f;
-								g[j] = bond_force_mixed<MODEL, VAR>(int_sub(x[j + 1], x[j], fj), fc, k1, s_tab, fj);
+								g[j] = bond_force_mixed<MODEL, VAR, (E >= 4)>(int_sub(x[j + 1], x[j], fj), fc, k1, s_tab, fj);
 							}
 							if (__any_sync(0xffffffffu, f.bad() | (fl & fe.bad()))) {
 #pragma unroll
@@ -392,8 +387,24 @@ __global__ void __launch_bounds__(kMaxThreads<MODEL, E, WIN>) real_move_kernel_t
 			}
 		}
 		};
-		if (G <= 32) integrate(std::true_type{});
-		else integrate(std::false_type{});
+		// Operations on the integer pipes from 4 sites per lane on.  Lanes of fewer sites are those of
+		// ensembles too small to fill the schedulers, or of short chains: with a warp or two per scheduler
+		// the two pipes hardly overlap (a warp issues in order) and an operation costs 75 clocks against 64
+		// (FPUT N = 64, 100 steps, one site per lane: 232 us for 96 chains with the FP64 pipe alone, 403 with
+		// both; 1024 chains 497 against 679).  Toda, with 12 operations a site, gains from two warps
+		// per SM on (a.mixed; N = 128, 512 chains: 1082 -> 958 us; N = 64, 96 chains: 419 against 560).
+		if constexpr (E >= 4) {
+			if (G <= 32) integrate(std::true_type{}, std::true_type{});
+			else integrate(std::false_type{}, std::true_type{});
+		} else {
+			if (MODEL == NLC_TODA && a.mixed) {
+				if (G <= 32) integrate(std::true_type{}, std::bool_constant<MODEL == NLC_TODA>{});
+				else integrate(std::false_type{}, std::bool_constant<MODEL == NLC_TODA>{});
+			} else {
+				if (G <= 32) integrate(std::true_type{}, std::false_type{});
+				else integrate(std::false_type{}, std::false_type{});
+			}
+		}
 
 		if (active) {
 			const bool open = seg & NLC_SEG_OPEN;
