@@ -10,10 +10,10 @@
 // projection (the reference's two cublasDgemm calls, dDNKG.cpp:118-133, plus dDNKG.cu:237-256).
 //
 // The sum over copies (the reference's MPI all_reduce, results_entropy.cpp:13) runs on the device
-// in a fixed order: each team (or, for dDNKG, each block) accumulates its chains into its own
-// partial row, and a single-block finish kernel sums the rows in row order, normalises, and
-// computes the WT / information entropies (results_entropy.cpp:21-46).  Results are therefore
-// identical from run to run on a given GPU.
+// in a fixed order: each team accumulates its chains, each block adds its teams into its own partial
+// row, and a finish kernel sums the rows in a fixed order, normalises, and computes the WT /
+// information entropies (results_entropy.cpp:21-46).  Results are therefore identical from run to
+// run on a given GPU.
 #include <algorithm>
 
 #include "nlc_fft.cuh"
@@ -30,8 +30,30 @@ __device__ __noinline__ double mode_energy_fp64(double ak, double bk, double2 zk
 }
 
 // One team (warp, or whole block when BLOCK) per chain; shared memory per team: 2 n complex
-// (ping-pong).  Each team accumulates its chains into its own row of `partials` (row = block *
-// teams + team), so no two threads ever add into the same element.
+// (ping-pong).  A block accumulates into its own row of `partials`: a team that is the whole block
+// in place, warp teams in a row of shared memory each, which the block adds in team order at its end
+// (a quarter of the rows for the finish to read, and no global reads and writes per chain).  No two
+// threads ever add into the same element.
+template <bool BLOCK>
+__device__ __forceinline__ double *team_row(const DiagArgs &a, double *rows, int team, int t, int T) {
+	const int n = int(a.n);
+	double *acc = BLOCK ? a.partials + (size_t) blockIdx.x * n : rows + (size_t) team * n;
+	for (int k = t; k < n; k += T) acc[k] = 0.;
+	return acc;
+}
+
+template <bool BLOCK>
+__device__ __forceinline__ void add_team_rows(const DiagArgs &a, const double *rows, int teams) {
+	if (BLOCK) return;
+	const int n = int(a.n);
+	__syncthreads();
+	for (int k = threadIdx.x; k < n; k += blockDim.x) {
+		double v = rows[k];
+		for (int q = 1; q < teams; q++) v = dadd(v, rows[(size_t) q * n + k]);
+		a.partials[(size_t) blockIdx.x * n + k] = v;
+	}
+}
+
 template <bool BLOCK>
 __global__ void __launch_bounds__(BLOCK ? 512 : 128) lin_fft_kernel(const double2 *__restrict__ state, const DiagArgs a) {
 	extern __shared__ double2 sm[];
@@ -43,8 +65,8 @@ __global__ void __launch_bounds__(BLOCK ? 512 : 128) lin_fft_kernel(const double
 	const int len = a.fft.len;
 	double2 *x = BLOCK && a.gscratch ? a.gscratch + (size_t) blockIdx.x * 2 * len : sm + (size_t) team * 2 * len;
 	double2 *y = x + len;
-	double *acc = a.partials + ((size_t) blockIdx.x * teams + team) * n;
-	for (int k = t; k < n; k += T) acc[k] = 0.;
+	double *const rows = reinterpret_cast<double *>(sm + (size_t) teams * 2 * len);
+	double *const acc = team_row<BLOCK>(a, rows, team, t, T);
 
 	const bool dnls = a.model == NLC_DNLS;
 	const FpOnes k1 = in_register(a.fft.k1, lane_zero(a.fft.k1));
@@ -88,6 +110,7 @@ __global__ void __launch_bounds__(BLOCK ? 512 : 128) lin_fft_kernel(const double
 		}
 		team_sync<BLOCK>();
 	}
+	add_team_rows<BLOCK>(a, rows, teams);
 }
 
 // The FP32 diagnostics (NLC_FLAG_FP32_DIAGNOSTICS): the same teams and partial rows, each chain
@@ -105,8 +128,8 @@ __global__ void __launch_bounds__(BLOCK ? 512 : 128) lin_fft32_kernel(const doub
 	const int len = a.fft.len;
 	float2 *x = smf + (size_t) team * 2 * len;
 	float2 *y = x + len;
-	double *acc = a.partials + ((size_t) blockIdx.x * teams + team) * n;
-	for (int k = t; k < n; k += T) acc[k] = 0.;
+	double *const rows = reinterpret_cast<double *>(smf + (size_t) teams * 2 * len);
+	double *const acc = team_row<BLOCK>(a, rows, team, t, T);
 	const bool dnls = a.model == NLC_DNLS;
 	for (unsigned long long chain = (unsigned long long) blockIdx.x * teams + team; chain < a.copies;
 	     chain += (unsigned long long) gridDim.x * teams) {
@@ -132,6 +155,7 @@ __global__ void __launch_bounds__(BLOCK ? 512 : 128) lin_fft32_kernel(const doub
 		}
 		team_sync<BLOCK>();
 	}
+	add_team_rows<BLOCK>(a, rows, teams);
 }
 
 // dDNKG projection: a block takes CH chains at a time; thread k of a block of modes accumulates
@@ -316,172 +340,117 @@ cudaError_t launch_initial_state(const DiagArgs &diag, const IcArgs &c, double2 
 cudaError_t launch_linenergies_partials(const DiagArgs &a, const void *state, int blocks, int threads,
                                         size_t smem, int team_block, cudaStream_t stream) {
 	const double2 *st = static_cast<const double2 *>(state);
+	const size_t rows = team_block || a.model == NLC_DDNKG ? 0 : threads / 32 * size_t(a.n) * sizeof(double);
 	count_launch();
 	if (a.model == NLC_DDNKG) {
 		lin_ddnkg_kernel<<<blocks, threads, smem, stream>>>(st, a);
 	} else if (a.tw32) {
 		if (team_block) lin_fft32_kernel<true><<<blocks, threads, smem / 2, stream>>>(st, a);
-		else lin_fft32_kernel<false><<<blocks, threads, smem / 2, stream>>>(st, a);
+		else lin_fft32_kernel<false><<<blocks, threads, smem / 2 + rows, stream>>>(st, a);
 	} else if (team_block) {
 		lin_fft_kernel<true><<<blocks, threads, smem, stream>>>(st, a);
 	} else {
-		lin_fft_kernel<false><<<blocks, threads, smem, stream>>>(st, a);
+		lin_fft_kernel<false><<<blocks, threads, smem + rows, stream>>>(st, a);
 	}
 	return cudaGetLastError();
 }
 
-// Single block: sum the partial rows in a fixed order, normalise, entropies.  For n <= 1024 the
-// rows are split into 1024/n interleaved slices (thread t: mode t % n, slice t / n, coalesced
-// reads), the slices are then added in slice order; the result is identical on every run.
-constexpr int kFinishThreads = 1024;
-
-__device__ __forceinline__ void finish_mode(const FinishArgs &a, int k, double v, double &se, double &sl,
-                                            double &sel, int &cnt) {
+// The sum of the partial rows, the normalisation and the entropies, in one launch.  A block takes
+// 8 or 16 modes (tile): its threads are slices of the rows by modes (64 or 128 bytes of a row each),
+// every slice adds its rows in row order, the slices are added in a fixed tree, and the block's
+// entropy sums {sum e, sum log e, sum e log e, count} go to block_sums; the last block to finish (a
+// counter, no waiting) adds those of all blocks in a fixed order.  The result is identical on every run.
+// What it costs is latency: the launches, the loads' round trips and the serial sums.  One launch with
+// eight loads in flight per thread and a row per block, against one launch for slices of the rows and
+// one or two to finish them over a row per team: a sample of 64 sites x 96 copies in a job with 100
+// steps 71.1 -> 66.7 us in all, 128 x 65536 336 -> 328 us, 512 x 64 48.6 -> 22.6 us, 4096 x 512
+// 221 -> 195 us.  Four to eight blocks of 1024 threads over a row per team instead take 9 us more than
+// those launches at 128 x 65536: a few SMs cannot draw 2 MB from L2 in that time.
+__device__ __forceinline__ void finish_mode(const FinishArgs &a, int k, double v, double &se, double &sl, double &sel,
+                                            double &cnt) {
 	if (a.model == NLC_DNLS) v = dmul(v, a.omega[k]);
 	if (a.a0is0 && k == 0) v = 0.;
 	v = dmul(v, a.norm);
 	a.lin[k] = v;
 	if ((!a.mask || a.mask[k]) && !(a.a0is0 && k == 0)) {
 		const double lv = log(v);
-		se = dadd(se, v), sl = dadd(sl, lv), sel = dfma(v, lv, sel);
-		cnt++;
+		se = v, sl = lv, sel = dmul(v, lv), cnt = 1.;
 	}
 }
 
-__global__ void __launch_bounds__(kFinishThreads) lin_finish_kernel(const FinishArgs a) {
-	__shared__ double r_e[kFinishThreads], r_l[kFinishThreads], r_el[kFinishThreads];
-	__shared__ int r_c[kFinishThreads];
-	const int t = threadIdx.x;
-	const int n = int(a.n);
-	double se = 0., sl = 0., sel = 0.;
-	int cnt = 0;
-	if (n <= kFinishThreads) {
-		const int slices = kFinishThreads / n;
-		const int k = t % n, sidx = t / n;
-		double v = 0.;
-		if (sidx < slices)
-			for (int r = sidx; r < a.nblocks; r += slices) v = dadd(v, a.partials[(size_t) r * n + k]);
-		r_e[t] = v;
-		__syncthreads();
-		if (t < n) {
-			double tot = 0.;
-			for (int q = 0; q < slices; q++) tot = dadd(tot, r_e[q * n + t]);
-			finish_mode(a, t, tot, se, sl, sel, cnt);
-		}
-		__syncthreads();
-	} else {
-		for (int k = t; k < n; k += kFinishThreads) {
-			double v = 0.;
-			for (int r = 0; r < a.nblocks; r++) v = dadd(v, a.partials[(size_t) r * n + k]);
-			finish_mode(a, k, v, se, sl, sel, cnt);
-		}
-	}
-	r_e[t] = se, r_l[t] = sl, r_el[t] = sel, r_c[t] = cnt;
-	__syncthreads();
-	for (int w = kFinishThreads / 2; w > 0; w >>= 1) {
-		if (t < w) {
-			r_e[t] = dadd(r_e[t], r_e[t + w]);
-			r_l[t] = dadd(r_l[t], r_l[t + w]);
-			r_el[t] = dadd(r_el[t], r_el[t + w]);
-			r_c[t] += r_c[t + w];
-		}
-		__syncthreads();
-	}
-	if (t == 0 && a.entropies) {
-		const double modes = r_c[0];
-		const double normalization = modes / r_e[0], lognorm = log(normalization);
-		a.entropies[0] = -(r_l[0] + modes * lognorm);
-		a.entropies[1] = normalization * (r_el[0] + lognorm * r_e[0]);
-	}
-}
+constexpr int kFinishThreads = 512;
 
-// Long chains: the row sums of 256 modes per block (coalesced over the modes, rows in order), the
-// normalisation and the block's entropy sums {sum e, sum log e, sum e log e, count} in a fixed
-// tree; then one block adds the blocks' sums in order and forms the entropies.
-__global__ void __launch_bounds__(kFinishModesPerBlock) lin_finish_modes_kernel(const FinishArgs a) {
-	__shared__ double r_e[kFinishModesPerBlock], r_l[kFinishModesPerBlock], r_el[kFinishModesPerBlock];
-	__shared__ int r_c[kFinishModesPerBlock];
-	const int t = threadIdx.x, k = blockIdx.x * kFinishModesPerBlock + t;
-	double se = 0., sl = 0., sel = 0.;
-	int cnt = 0;
-	if (k < (int) a.n) {
-		double v = 0.;
-		for (int r = 0; r < a.nblocks; r++) v = dadd(v, a.partials[(size_t) r * a.n + k]);
-		finish_mode(a, k, v, se, sl, sel, cnt);
-	}
-	r_e[t] = se, r_l[t] = sl, r_el[t] = sel, r_c[t] = cnt;
-	__syncthreads();
-	for (int w = kFinishModesPerBlock / 2; w > 0; w >>= 1) {
-		if (t < w) {
-			r_e[t] = dadd(r_e[t], r_e[t + w]);
-			r_l[t] = dadd(r_l[t], r_l[t + w]);
-			r_el[t] = dadd(r_el[t], r_el[t + w]);
-			r_c[t] += r_c[t + w];
-		}
-		__syncthreads();
-	}
-	if (t == 0) {
-		double *o = a.block_sums + 4 * (size_t) blockIdx.x;
-		o[0] = r_e[0], o[1] = r_l[0], o[2] = r_el[0], o[3] = r_c[0];
-	}
-}
-
-__global__ void lin_finish_entropy_kernel(const FinishArgs a, int blocks) {
-	if (threadIdx.x != 0 || !a.entropies) return;
-	double se = 0., sl = 0., sel = 0., modes = 0.;
-	for (int b = 0; b < blocks; b++) {
-		const double *o = a.block_sums + 4 * (size_t) b;
-		se = dadd(se, o[0]), sl = dadd(sl, o[1]), sel = dadd(sel, o[2]), modes = dadd(modes, o[3]);
-	}
-	const double normalization = modes / se, lognorm = log(normalization);
-	a.entropies[0] = -(sl + modes * lognorm);
-	a.entropies[1] = normalization * (sel + lognorm * se);
-}
-
-// Pre-reduction of many partial rows: block (x, y) adds rows [y per_slice, (y + 1) per_slice) of
-// the modes of tile x in row order, so that the finish reads one row per slice.  Every sum keeps a
-// fixed order: the result is identical on every run.
-__global__ void lin_rows_kernel(const double *__restrict__ partials, int rows, uint32_t n, int per_slice,
-                                double *__restrict__ out) {
-	const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
-	if (k >= n) return;
-	const int r0 = int(blockIdx.y) * per_slice, r1 = min(rows, r0 + per_slice);
+__global__ void __launch_bounds__(kFinishThreads) lin_finish_kernel(const FinishArgs a, int tile) {
+	__shared__ double part[kFinishThreads];
+	__shared__ double warp_sums[4][32];
+	__shared__ bool last;
+	const int tid = threadIdx.x, m = tid % tile, slice = tid / tile, slices = blockDim.x / tile;
+	const int n = int(a.n), k = blockIdx.x * tile + m;
 	double v = 0.;
-	for (int r = r0; r < r1; r++) v = dadd(v, partials[(size_t) r * n + k]);
-	out[(size_t) blockIdx.y * n + k] = v;
+	if (k < n) {
+		int r = slice;
+		for (; r + 7 * slices < a.nblocks; r += 8 * slices) {   // eight loads in flight, added in row order
+			double w[8];
+#pragma unroll
+			for (int i = 0; i < 8; i++) w[i] = a.partials[size_t(r + i * slices) * n + k];
+#pragma unroll
+			for (int i = 0; i < 8; i++) v = dadd(v, w[i]);
+		}
+		for (; r < a.nblocks; r += slices) v = dadd(v, a.partials[size_t(r) * n + k]);
+	}
+	part[tid] = v;
+	__syncthreads();
+	for (int w = blockDim.x / 2; w >= tile; w >>= 1) {
+		if (tid < w) part[tid] = dadd(part[tid], part[tid + w]);
+		__syncthreads();
+	}
+	double s[4] = {0., 0., 0., 0.};
+	if (tid < 32) {
+		if (tid < tile && k < n) finish_mode(a, k, part[tid], s[0], s[1], s[2], s[3]);
+		for (int o = tile / 2; o > 0; o >>= 1)
+#pragma unroll
+			for (int i = 0; i < 4; i++) s[i] = dadd(s[i], __shfl_xor_sync(0xffffffffu, s[i], o));
+	}
+	if (!a.entropies) return;
+	if (tid == 0) {
+#pragma unroll
+		for (int i = 0; i < 4; i++) __stcg(a.block_sums + 4 * size_t(blockIdx.x) + i, s[i]);
+		__threadfence();
+		last = atomicInc(a.counter, gridDim.x - 1) == gridDim.x - 1;   // back to zero by itself
+	}
+	__syncthreads();
+	if (!last) return;
+	__threadfence();
+#pragma unroll
+	for (int i = 0; i < 4; i++) s[i] = 0.;
+	for (int b = tid; b < int(gridDim.x); b += blockDim.x)
+#pragma unroll
+		for (int i = 0; i < 4; i++) s[i] = dadd(s[i], __ldcg(a.block_sums + 4 * size_t(b) + i));
+	const int warps = blockDim.x / 32;
+	for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+		for (int i = 0; i < 4; i++) s[i] = dadd(s[i], __shfl_xor_sync(0xffffffffu, s[i], o));
+	if (tid % 32 == 0)
+#pragma unroll
+		for (int i = 0; i < 4; i++) warp_sums[i][tid / 32] = s[i];
+	__syncthreads();
+	if (tid == 0) {
+		for (int w = 1; w < warps; w++)
+#pragma unroll
+			for (int i = 0; i < 4; i++) s[i] = dadd(s[i], warp_sums[i][w]);
+		const double normalization = s[3] / s[0], lognorm = log(normalization);
+		a.entropies[0] = -(s[1] + s[3] * lognorm);
+		a.entropies[1] = normalization * (s[2] + lognorm * s[0]);
+	}
 }
 
-constexpr int kRowsPerSliceMin = 8;
-
-int finish_row_slices(uint32_t n, int rows, int sms) {
-	if (rows < 8 * kRowsPerSliceMin) return 0;
-	const int tiles = int((n + kFinishModesPerBlock - 1) / kFinishModesPerBlock);
-	const int want = (2 * sms + tiles - 1) / tiles;   // about two blocks per SM
-	const int slices = std::min(want, (rows + kRowsPerSliceMin - 1) / kRowsPerSliceMin);
-	return slices >= 2 ? slices : 0;
-}
-
-cudaError_t launch_linenergies_finish(const FinishArgs &in, cudaStream_t stream) {
-	FinishArgs a = in;
-	if (a.row_slices && a.row_slice_cap >= 2 && a.nblocks >= 8 * kRowsPerSliceMin) {
-		const int per_slice = (a.nblocks + a.row_slice_cap - 1) / a.row_slice_cap;
-		const int slices = (a.nblocks + per_slice - 1) / per_slice;
-		const int threads = int(std::min<uint32_t>(kFinishModesPerBlock, (a.n + 31) / 32 * 32));
-		count_launch();
-		lin_rows_kernel<<<dim3((a.n + threads - 1) / threads, slices), threads, 0, stream>>>(a.partials, a.nblocks, a.n,
-		                                                                                   per_slice, a.row_slices);
-		a.partials = a.row_slices;
-		a.nblocks = slices;
-	}
-	if (a.block_sums && a.n > (uint32_t) kFinishModesPerBlock) {
-		const int blocks = int((a.n + kFinishModesPerBlock - 1) / kFinishModesPerBlock);
-		count_launch(2);
-		lin_finish_modes_kernel<<<blocks, kFinishModesPerBlock, 0, stream>>>(a);
-		lin_finish_entropy_kernel<<<1, 32, 0, stream>>>(a, blocks);
-		return cudaGetLastError();
-	}
+cudaError_t launch_linenergies_finish(const FinishArgs &a, cudaStream_t stream) {
+	// about four rows per slice (a power of two of slices)
+	const int tile = finish_tile(a.n);
+	int threads = 32;
+	while (threads < kFinishThreads && 4 * (threads / tile) < a.nblocks) threads <<= 1;
 	count_launch();
-	lin_finish_kernel<<<1, kFinishThreads, 0, stream>>>(a);
+	lin_finish_kernel<<<finish_blocks(a.n), threads, 0, stream>>>(a, tile);
 	return cudaGetLastError();
 }
 

@@ -221,16 +221,12 @@ struct FinishArgs {
 	const uint8_t *mask;      // device, NULL = all modes
 	double *lin;              // out [n]
 	double *entropies;        // out [2] or NULL
-	double *block_sums;       // [ceil(n / 256)][4] scratch: with it, chains longer than 256 sites
-	                          // are finished by a grid over the modes instead of one block
-	double *row_slices;       // [row_slice_cap][n] scratch: with it, many partial rows are first
-	int row_slice_cap;        // added in slices by a grid over (mode tiles x slices)
+	double *block_sums;       // [finish_blocks(n)][4] scratch
+	unsigned int *counter;    // finished blocks (device, zero before a launch and after it)
 };
-// slices of the partial rows for a finish of n modes over `rows` rows on `sms` SMs: 0 when the
-// rows go to the finish directly
-int finish_row_slices(uint32_t n, int rows, int sms);
+inline int finish_tile(uint32_t n) { return n <= 512 ? 8 : 16; }   // modes per block of the finish
+inline unsigned finish_blocks(uint32_t n) { return (n + finish_tile(n) - 1) / finish_tile(n); }
 cudaError_t launch_linenergies_finish(const FinishArgs &a, cudaStream_t stream);
-constexpr int kFinishModesPerBlock = 256;
 
 // DNLS ------------------------------------------------------------------------------------------
 

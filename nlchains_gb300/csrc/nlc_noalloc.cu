@@ -48,12 +48,13 @@ DeviceSetup g_setup[kMaxDevices];
 
 // twiddles exp(-2 pi i e/n), the FMA-form twiddle entries of the radix-2/3/4 passes (entry e of
 // every pass after more than e points) and the per-mode coefficients: (omega+1)/2, (omega-1)/2 for
-// the real models, omega for DNLS (omega as in DNKG_FPUT_Toda/dispersion.cpp:9-16,
+// the real models, omega for DNLS; and the finish's counter (omega as in DNKG_FPUT_Toda/dispersion.cpp:9-16,
 // DNLS/dispersion.cpp:10-17)
 __global__ void noalloc_tables_kernel(uint32_t n, int model, double m, const FftPlanDev f, double2 *tw, double2 *gw,
-                                      double *ca, double *cb) {
+                                      double *ca, double *cb, unsigned int *counter) {
 	const uint32_t e = blockIdx.x * blockDim.x + threadIdx.x;
 	if (e >= n) return;
+	if (e == 0) *counter = 0;
 	double s, c;
 	sincospi(2. * e / n, &s, &c);
 	tw[e] = make_double2(c, -s);
@@ -174,20 +175,24 @@ extern "C" int nlc_linenergies_noalloc(int32_t model, uint32_t chain_length, uin
 			ns *= (unsigned long long) g.fft.radix[r];
 		}
 	}
-	// scratch layout: [twiddles 2n][FMA-form twiddles 6n][coef a n][coef b n][partial rows rows x n]
+	// scratch layout: [twiddles 2n][FMA-form twiddles 6n][coef a n][coef b n][entropy sums of the finish's
+	// blocks][its counter][partial rows rows x n]
 	double *base = S->scratch;
 	double2 *tw = reinterpret_cast<double2 *>(base);
 	double2 *gw = tw + n;
 	double *ca = base + 8 * size_t(n), *cb = ca + n;
-	double *rows_base = cb + n;
-	const size_t rows_cap = (kNoAllocScratchDoubles - 10 * size_t(n)) / n;
-	const int team_block = n > 1024;
+	double *sums = cb + n;
+	unsigned int *counter = reinterpret_cast<unsigned int *>(sums + 4 * size_t(finish_blocks(n)));
+	double *rows_base = sums + 4 * size_t(finish_blocks(n)) + 2;
+	const size_t rows_cap = (kNoAllocScratchDoubles - size_t(rows_base - base)) / n;
+	// the teams of a plan's diagnostics (512 sites x 4096 copies: 174 us, 378 with a warp per chain)
+	const int team_block = n > 256;
 	const int teams = team_block ? 1 : 4;
-	const int threads = team_block ? 256 : 128;
+	const int threads = team_block ? (n <= 512 ? 64 : n <= 1024 ? 128 : 256) : 128;
 	const size_t smem = size_t(teams) * 2 * n * sizeof(double2);
 	unsigned long long blocks = (copies + teams - 1) / teams;
-	blocks = std::min<unsigned long long>(blocks, 4ull * S->sms);
-	blocks = std::min<unsigned long long>(blocks, rows_cap / teams);
+	blocks = std::min<unsigned long long>(blocks, (512ull / threads) * S->sms);   // as many as the registers hold
+	blocks = std::min<unsigned long long>(blocks, rows_cap);
 	if (!blocks) return set_error(NLC_EINVAL, "nlc_linenergies_noalloc: scratch too small for this chain_length");
 	g.fft.tw = tw;
 	g.fft.gw = gw;
@@ -197,14 +202,15 @@ extern "C" int nlc_linenergies_noalloc(int32_t model, uint32_t chain_length, uin
 
 	cudaStream_t st = static_cast<cudaStream_t>(stream);
 	count_launch();
-	noalloc_tables_kernel<<<(n + 127) / 128, 128, 0, st>>>(n, model, model == NLC_DNKG ? m : 0., g.fft, tw, gw, ca, cb);
+	noalloc_tables_kernel<<<(n + 127) / 128, 128, 0, st>>>(n, model, model == NLC_DNKG ? m : 0., g.fft, tw, gw, ca, cb,
+	                                                       counter);
 	if ((rc = cuda_status(cudaGetLastError(), "nlc_linenergies_noalloc tables launch"))) return rc;
 	if ((rc = cuda_status(launch_linenergies_partials(g, state_dev, int(blocks), threads, smem, team_block, st),
 	                      "nlc_linenergies_noalloc launch")))
 		return rc;
 	FinishArgs f{};
 	f.partials = rows_base;
-	f.nblocks = int(blocks) * teams;
+	f.nblocks = int(blocks);
 	f.n = n;
 	// normalisations of results::calc_linenergies (DNKG_FPUT_Toda.cpp:129, DNLS.cpp:150) and a0is0
 	f.norm = model == NLC_DNLS ? 1. / (double(copies) * n) : (0.5 / copies) / n;
@@ -214,5 +220,7 @@ extern "C" int nlc_linenergies_noalloc(int32_t model, uint32_t chain_length, uin
 	f.mask = entropy_mask_dev;
 	f.lin = lin_dev;
 	f.entropies = entropies_dev;
+	f.block_sums = sums;
+	f.counter = counter;
 	return cuda_status(launch_linenergies_finish(f, st), "nlc_linenergies_noalloc finish launch");
 }

@@ -112,9 +112,7 @@ struct nlc_plan {
 	size_t device_bytes = 0;
 	unsigned long long *d_counter = nullptr;
 	double *d_partials = nullptr;
-	double *d_row_slices = nullptr;   // pre-reduced partial rows (finish_row_slices)
-	int row_slice_cap = 0;
-	double *d_block_sums = nullptr;   // entropy sums of the mode blocks (chains above 256 sites)
+	double *d_block_sums = nullptr;   // entropy sums of the finish's blocks
 	uint8_t *d_mask = nullptr;
 
 	RealArgs ra{};
@@ -655,7 +653,7 @@ int setup_diagnostics(nlc_plan &P) {
 			P.diag_smem = size_t(teams) * 2 * len * sizeof(double2);
 			const unsigned long long groups = (P.m.copies + teams - 1) / teams;
 			P.diag_blocks = int(std::min<unsigned long long>(groups, (compact ? 1ull : 4ull) * sms));
-			P.diag_rows = P.diag_blocks * teams;
+			P.diag_rows = P.diag_blocks;
 		} else {
 			// A block per chain: the chain's two buffers in shared memory bound the chains per SM, so the
 			// threads per chain are what fills the schedulers (the fastest of 32 .. 512 at each length:
@@ -681,7 +679,7 @@ int setup_diagnostics(nlc_plan &P) {
 				if ((rc = P.dalloc(&g.gscratch, size_t(P.diag_blocks) * 2 * len))) return rc;
 			}
 		}
-		g.mixed = (unsigned long long) P.diag_rows * (P.diag_team_block ? P.diag_threads / 32 : 1) >= 8ull * sms;
+		g.mixed = (unsigned long long) P.diag_blocks * (P.diag_threads / 32) >= 8ull * sms;
 		if (!g.mixed) g.fft.fp64_first = 1;
 		// FP32 diagnostics: for direct transforms held in shared memory (padded lengths and
 		// global-memory passes keep the FP64 transform)
@@ -706,11 +704,7 @@ int setup_diagnostics(nlc_plan &P) {
 		return set_error(NLC_EUNSUPPORTED, "chain_length too large for the shared-memory diagnostics");
 	if ((rc = P.dalloc(&P.d_partials, size_t(P.diag_rows) * n))) return rc;
 	g.partials = P.d_partials;
-	P.row_slice_cap = finish_row_slices(n, P.diag_rows, sms);
-	if (P.row_slice_cap && (rc = P.dalloc(&P.d_row_slices, size_t(P.row_slice_cap) * n))) return rc;
-	if (n > uint32_t(kFinishModesPerBlock) &&
-	    (rc = P.dalloc(&P.d_block_sums, 4 * size_t((n + kFinishModesPerBlock - 1) / kFinishModesPerBlock))))
-		return rc;
+	if ((rc = P.dalloc(&P.d_block_sums, 4 * size_t(finish_blocks(n))))) return rc;
 	if (!P.mask_host.empty()) {
 		if ((rc = P.upload(&P.d_mask, P.mask_host.data(), n))) return rc;
 	}
@@ -971,8 +965,8 @@ extern "C" int nlc_plan_create(const nlc_model *model, nlc_plan **out) {
 	}
 
 	{   // zeroed by a copy, not a memset kernel, so that plan creation needs no free SM
-		const unsigned long long zero[2] = {0, 0};
-		if ((rc = P->upload(&P->d_counter, zero, 2))) return rc;
+		const unsigned long long zero[3] = {0, 0, 0};   // the integrator's two, the finish's
+		if ((rc = P->upload(&P->d_counter, zero, 3))) return rc;
 	}
 
 	if (mdl == NLC_DNLS) {
@@ -1431,8 +1425,7 @@ extern "C" int nlc_linenergies(nlc_plan *P, const void *state, double *lin, doub
 	f.lin = lin;
 	f.entropies = ent;
 	f.block_sums = P->d_block_sums;
-	f.row_slices = P->d_row_slices;
-	f.row_slice_cap = P->row_slice_cap;
+	f.counter = reinterpret_cast<unsigned int *>(P->d_counter + 2);
 	return cuda_status(launch_linenergies_finish(f, st), "linenergies finish launch");
 }
 
