@@ -313,11 +313,17 @@ struct TcArgs {
 	const int *col_exp;        // [n] exponent of each eigenvector (row of E)
 	const double *omega;       // [n]
 	double *partials;          // [mp / 128][n] weighted squared sums per row tile
-	long long *park;           // [mp][np] the hi sums of the first sweep (7 slices only)
+	int whole, parts;          // tiles taken by one block each, blocks per tile of the rest
+	long long *park;           // [blocks][128][128] the hi sums of the first sweep (7 slices only)
+	long long *part_sums;      // [blocks of the rest][128][128] their sums (parts > 1)
+	unsigned int *part_count;  // [tiles of the rest] finished parts (zero between launches)
+	int *part_fail;            // [tiles of the rest] a part gave up (zero between launches)
 	int *status;               // set on a bounded-wait timeout
 	unsigned long long wait_ns;  // limit of every mbarrier wait (wall clock)
 	int wait_test;             // tests only: thread 0 first waits on a barrier nothing arrives at
 };
+inline size_t tc_projection_tiles(const TcArgs &a) { return size_t(a.mp / 128) * (a.np / 128); }
+inline size_t tc_projection_blocks(const TcArgs &a) { return a.whole + (tc_projection_tiles(a) - a.whole) * a.parts; }
 cudaError_t launch_tc_projection(const TcArgs &a, const double2 *state, cudaStream_t stream);
 size_t tc_projection_smem(int slices);
 const void *tc_projection_kernel_ptr(int slices);

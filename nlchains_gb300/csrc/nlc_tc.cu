@@ -186,6 +186,19 @@ __device__ __forceinline__ void issue_sweep_mmas(uint32_t tmem, uint64_t da, uin
 	}
 }
 
+// The integer in an FP32 accumulator (|v| <= 2^26) without a conversion instruction: v = 4096 h + l
+// with h and l rounded into the low bits of 1.5 2^23 + h and 1.5 2^23 + l (all steps exact).
+// Conversions issue at 16 lanes a clock and took most of the read-out's time; half of the values
+// take this form, six instructions of pipes that the read-out leaves idle (1024 x 4096: with the
+// epilogue's 32-bit conversion 429 -> 403 us).
+__device__ __forceinline__ int group_sum_fp32(uint32_t bits) {
+	constexpr float kRound = 12582912.f;   // 1.5 2^23
+	constexpr uint32_t kBits = 0x4b400000u;
+	const float v = __uint_as_float(bits), h = __fmaf_rn(v, 1.f / 4096.f, kRound);
+	const float l = __fadd_rn(__fmaf_rn(__fsub_rn(h, kRound), -4096.f, v), kRound);
+	return (int) (__float_as_uint(h) * 4096u + __float_as_uint(l) - kBits * 4097u);
+}
+
 }  // namespace
 
 // 7 balanced base-256 digits of x 2^(56 - e) (e: the row exponent, |x| < 2^e), in integer
@@ -259,16 +272,25 @@ __global__ void tc_split_rows_kernel(const double2 *__restrict__ state, TcArgs a
 	const int ephi = row_exp(mphi), epi = row_exp(mpi);
 	const unsigned long long r = 2 * c;
 	if (lane == 0) a.row_exp[r] = ephi, a.row_exp[r + 1] = epi;
-	for (uint32_t s = lane; s < n; s += 32) {
-		const double2 v = chain[s];
-		uint16_t sp[7], sq[7];
-		split7(v.x, ephi, sp);
-		split7(v.y, epi, sq);
+	// four sites per lane: eight bytes of a slice's row per store (1024 sites x 4096 chains 46 us, with a
+	// site per lane 53; bound by the integer instructions, about 60 a value)
+	for (uint32_t s = 4 * lane; s < n; s += 128) {
+		double2 v[4];
+#pragma unroll
+		for (int j = 0; j < 4; j++) v[j] = s + j < n ? chain[s + j] : make_double2(0., 0.);
 		// slice i lies 128 x 16 elements after slice i - 1; rows 2c and 2c + 1 share a tile and a
 		// swizzle phase, so the pi row is the phi row's position plus one row
 		uint16_t *dst = a.a_slices + tc_slice_index(0, (int) (s >> 4), a.mp, r, (int) (s & 15), S);
+		uint16_t sl[4][7];
 #pragma unroll
-		for (int i = 0; i < S; i++) dst[i * 128 * 16] = sp[i], dst[i * 128 * 16 + 16] = sq[i];
+		for (int q = 0; q < 2; q++) {
+#pragma unroll
+			for (int j = 0; j < 4; j++) split7(q ? v[j].y : v[j].x, q ? epi : ephi, sl[j]);
+#pragma unroll
+			for (int i = 0; i < S; i++)
+				*reinterpret_cast<uint2 *>(dst + i * 128 * 16 + 16 * q) =
+				    make_uint2(sl[0][i] | (uint32_t) sl[1][i] << 16, sl[2][i] | (uint32_t) sl[3][i] << 16);
+		}
 	}
 }
 
@@ -291,7 +313,7 @@ tc_projection_kernel(const TcArgs a) {
 	constexpr int kBarAcc = 2 * (kS0 + kS1), kBars = kBarAcc + 2;
 	__shared__ __align__(8) unsigned long long bars[kBars];
 	__shared__ uint32_t tmem_slot;
-	__shared__ int s_fail, s_issued;
+	__shared__ int s_fail, s_issued, s_finish, s_bad;
 	__shared__ double s_w[kBN];   // per column of the tile: omega_k^2 (weight of the phi rows)
 	__shared__ int s_cexp[kBN];   // per column: the eigenvector's power-of-two exponent
 	const int tid = threadIdx.x, warp = tid >> 5;
@@ -299,7 +321,12 @@ tc_projection_kernel(const TcArgs a) {
 	const int part = warp >> 2;                    // its columns: [kCols part, kCols (part + 1))
 	// tiles numbered with the column tiles fastest (see the header)
 	const int col_tiles = a.np / kBN;
-	const int row_tile = (int) (blockIdx.x / col_tiles), col_tile = (int) (blockIdx.x % col_tiles);
+	// a block takes a whole tile, or (the last tiles) one of a.parts parts of its chunks of K
+	const int split = (int) blockIdx.x - a.whole;   // index among the blocks that take parts
+	const int parts = split < 0 ? 1 : a.parts;
+	const int tail = split < 0 ? 0 : split / parts, slice_of_k = split < 0 ? 0 : split % parts;
+	const int tile = split < 0 ? (int) blockIdx.x : a.whole + tail;
+	const int row_tile = tile / col_tiles, col_tile = tile % col_tiles;
 	const int row0 = row_tile * kBM, col0 = col_tile * kBN;
 	const uint32_t accb = smem_u32(&bars[kBarAcc]);
 	if (tid == 0) {
@@ -329,7 +356,11 @@ tc_projection_kernel(const TcArgs a) {
 	asm volatile("tcgen05.fence::after_thread_sync;");
 	const uint32_t tmem = tmem_slot;
 
-	const int nkb = a.kp / kBK;   // 16-site blocks of K
+	// this block's 16-site blocks of K: kb0 .. kb0 + nkb, whole chunks
+	constexpr int kChunkBlocks = kChunkK / kBK;
+	const int chunks = (a.kp / kBK + kChunkBlocks - 1) / kChunkBlocks;
+	const int kb0 = slice_of_k * chunks / parts * kChunkBlocks;
+	const int nkb = min(a.kp / kBK, (slice_of_k + 1) * chunks / parts * kChunkBlocks) - kb0;
 	// the MMA threads' bookkeeping for the failure path: the sweep's barriers and stage count, stages
 	// landed (the producer's loads: s_issued), and whether the current chunk's MMAs are committed
 	uint32_t cur_full = smem_u32(&bars[kBarFull0]);
@@ -361,7 +392,7 @@ tc_projection_kernel(const TcArgs a) {
 			asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(full), "r"(blocks * kBlockBytes) : "memory");
 			unsigned char *base = stage_ptr(s);
 			for (int b = 0; b < blocks; b++) {
-				const int kb = it * KB + b;
+				const int kb = kb0 + it * KB + b;
 				unsigned char *blk = base + (size_t) b * kBlockBytes;
 				bulk_load(smem_u32(blk), a.a_slices + tc_slice_index(0, kb, a.mp, row0, 0, S), NS * kTile, full);
 				bulk_load(smem_u32(blk + (size_t) NS * kTile), a.b_slices + tc_slice_index(0, kb, a.np, col0, 0, S), NS * kTile,
@@ -442,8 +473,7 @@ tc_projection_kernel(const TcArgs a) {
 						const int shift = W == 0 ? (g == 0 ? 16 : g == 1 ? 8 : 0) : 8 * (3 - g);
 #pragma unroll
 						for (int j = 0; j < 8; j++) {
-							const long long gv = __float2int_rn(__uint_as_float(v[q][j]));   // below 2^26: a 32-bit conversion
-							acc[sg * 8 + j] += gv << shift;
+							acc[sg * 8 + j] += (long long) (j & 1 ? group_sum_fp32(v[q][j]) : __float2int_rn(__uint_as_float(v[q][j]))) << shift;
 						}
 					}
 				}
@@ -456,13 +486,48 @@ tc_projection_kernel(const TcArgs a) {
 
 	// parked hi sums of this thread, column-major within the tile ([col][row]): the 32 threads of a
 	// warp, 32 consecutive rows, store and load 256 contiguous bytes per column
-	long long *park = a.park + ((size_t) blockIdx.x * kBN + part * kCols) * kBM + rl;
+	const size_t mine = (size_t) part * kCols * kBM + rl;
+	auto park_of = [&](int block) { return a.park + (size_t) block * (kBN * kBM) + mine; };
 	sweep(std::integral_constant<int, 0>{});
 	if constexpr (S == kSlicesFull) {
 		if (!s_fail) {
+			long long *park = park_of((int) blockIdx.x);
 #pragma unroll
 			for (int c = 0; c < kCols; c++) park[c * kBM] = acc[c], acc[c] = 0;
 			sweep(std::integral_constant<int, 1>{});
+		}
+	}
+
+	// A tile in parts: every block leaves its sums, and the last one to do so (a counter, no waiting)
+	// adds the others' and finishes the tile.  The sums are exact integers: the same in any order.
+	bool finish = true, bad = s_fail;
+	if (parts > 1) {
+		long long *const sums = a.part_sums + (size_t) split * (kBN * kBM) + mine;
+		if (!bad) {
+#pragma unroll
+			for (int c = 0; c < kCols; c++) __stcg(sums + c * kBM, acc[c]);
+		}
+		__threadfence();
+		__syncthreads();
+		if (tid == 0) {
+			if (bad) {
+				atomicExch(a.part_fail + tail, 1);
+				__threadfence();
+			}
+			s_finish = atomicInc(a.part_count + tail, parts - 1) == (unsigned) (parts - 1);
+			__threadfence();
+			s_bad = s_finish ? atomicExch(a.part_fail + tail, 0) : 0;
+		}
+		__syncthreads();
+		finish = s_finish, bad = bad || s_bad;
+		if (finish && !bad) {
+			__threadfence();
+			for (int p = 0; p < parts; p++) {
+				if (p == slice_of_k) continue;
+				const long long *o = a.part_sums + (size_t) (tail * parts + p) * (kBN * kBM) + mine;
+#pragma unroll
+				for (int c = 0; c < kCols; c++) acc[c] += __ldcg(o + c * kBM);
+			}
 		}
 	}
 
@@ -478,14 +543,21 @@ tc_projection_kernel(const TcArgs a) {
 	static_assert(kThreads == 4 * kBN, "four threads per column");
 	const int r = row0 + rl;
 	const int er = r < 2 * (int) a.copies ? a.row_exp[r] : 0;
-	if (!s_fail) {
+	if (finish && !bad) {
 		// eight columns at a time: their parked sums loaded together, so a warp waits for L2 once per
 		// eight columns rather than once per column
 #pragma unroll
 		for (int c0 = 0; c0 < kCols; c0 += 8) {
 			long long hv[8];
 #pragma unroll
-			for (int j = 0; j < 8; j++) hv[j] = S == kSlicesFull ? __ldcg(park + (c0 + j) * kBM) : acc[c0 + j];
+			for (int j = 0; j < 8; j++) hv[j] = S == kSlicesFull ? 0 : acc[c0 + j];
+			if constexpr (S == kSlicesFull) {
+				for (int p = 0; p < parts; p++) {
+					const long long *park = park_of(split < 0 ? tile : a.whole + tail * parts + p);
+#pragma unroll
+					for (int j = 0; j < 8; j++) hv[j] += __ldcg(park + (c0 + j) * kBM);
+				}
+			}
 #pragma unroll
 			for (int j = 0; j < 8; j++) {
 				const int c = c0 + j, col = part * kCols + c;
@@ -500,7 +572,7 @@ tc_projection_kernel(const TcArgs a) {
 		}
 	}
 	__syncthreads();
-	{
+	if (finish) {
 		// rows 32 q .. 32 q + 31 of column tid mod 128; rows 0 and 2 mod 4 are phi rows
 		const int cc = tid & (kBN - 1), q = tid >> 7;
 		const double *col = red + cc * kRedStride + 32 * q;
@@ -510,12 +582,12 @@ tc_projection_kernel(const TcArgs a) {
 		quarter[q * kBN + cc] = make_double2(s0 + s2, s1 + s3);
 	}
 	__syncthreads();
-	if (tid < kBN) {
+	if (finish && tid < kBN) {
 		const int k = col0 + tid;
 		if (k < (int) a.n) {
 			const double2 q0 = quarter[tid], q1 = quarter[kBN + tid], q2 = quarter[2 * kBN + tid], q3 = quarter[3 * kBN + tid];
 			const double e = s_w[tid] * ((q0.x + q1.x) + (q2.x + q3.x)) + ((q0.y + q1.y) + (q2.y + q3.y));
-			a.partials[(size_t) row_tile * a.n + k] = s_fail ? __longlong_as_double(0x7ff8000000000000ll) : e;
+			a.partials[(size_t) row_tile * a.n + k] = bad ? __longlong_as_double(0x7ff8000000000000ll) : e;
 		}
 	}
 	if (s_fail) {
@@ -542,7 +614,7 @@ size_t tc_projection_smem(int) { return kStageMem + 1024; }
 
 cudaError_t launch_tc_projection(const TcArgs &a, const double2 *state, cudaStream_t stream) {
 	count_launch(2);
-	const dim3 grid((unsigned) ((size_t) (a.mp / kBM) * (a.np / kBN)));
+	const dim3 grid((unsigned) tc_projection_blocks(a));
 	const unsigned split_blocks = (unsigned) ((a.copies + 7) / 8);
 	if (a.slices == 3) {
 		tc_split_rows_kernel<3><<<split_blocks, 256, 0, stream>>>(state, a);

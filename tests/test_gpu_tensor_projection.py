@@ -118,3 +118,17 @@ def test_projection_wait_timeout_reported(gpu, monkeypatch, n, copies):
     bad.close()
     good.close()
     ctx.close()
+
+
+# tiles shared by several blocks: 300 x 3300 has 156 tiles, a full wave of 152 and 4 in two parts; 1030 x 200
+# 36 tiles with five chunks of K in four parts; 513 x 64 five tiles in three parts, the last of 16 sites
+@pytest.mark.parametrize("n,copies", [(300, 3300), (1030, 200), (513, 64)])
+def test_tensor_projection_in_parts(gpu, n, copies):
+    masses = ic.masses_uniform(n, seed=n)
+    state = np.random.default_rng(n + copies).standard_normal((copies, n, 2))
+    l64, w64, i64 = lin_of(gpu, n, copies, state, masses, gpu.FLAG_FP64_PROJECTION)
+    ltc, wtc, itc = lin_of(gpu, n, copies, state, masses, gpu.FLAG_TENSOR_PROJECTION)
+    assert np.abs(ltc - l64).max() <= 1e-13 * np.abs(l64).max()
+    assert abs(wtc - w64) <= 1e-12 * max(1.0, abs(w64)) and abs(itc - i64) <= 1e-12 * max(1.0, abs(i64))
+    l3, _, _ = lin_of(gpu, n, copies, state, masses, gpu.FLAG_BF16X3_PROJECTION)
+    assert np.abs(l3 - l64).max() <= 1e-6 * np.abs(l64).max()
