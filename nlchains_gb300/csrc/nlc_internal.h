@@ -89,7 +89,7 @@ struct RealArgs {
 	uint32_t copies;
 	uint32_t steps;
 	int32_t lanes;         // G: lanes per chain (power of two)
-	int32_t mixed;         // Toda: 1: integer-pipe operations on lanes of up to 3 sites too (more: always)
+	int32_t mixed;         // 1: integer-pipe operations on lanes of up to 3 sites too (more: always)
 	FpOnes k1;
 	ExpConsts ek;
 	// batched launch: when `batch` is set, the launch integrates every ensemble of the table (same

@@ -221,6 +221,18 @@ bool finish_shape(const nlc_plan &P, int model, int variant, RealShape &s, int t
 	return s.blocks > 0;
 }
 
+// Whether lanes of up to 3 sites have operations on the integer pipes (lanes of more always have): with
+// w warps per scheduler, an operation there has 75 clocks of latency and as many of its pipe against 64
+// on the FP64 pipe, so the two have to overlap.  Toda, with 12 operations a site, from w = 1/2 on (N = 128,
+// 512 chains: 1082 -> 892 us for 100 steps; N = 64, 96 chains: 419 against 560).  The others from w = 3 with
+// one site per lane, 1.5 with two (100 steps, FP64 pipe alone -> both: one site, DNKG 128 x 512 484 -> 444 us,
+// FPUT 64 x 1024 500 -> 493, 64 x 600 (w = 2) 304 -> 318; two sites, DNKG 128 x 1500 1177 -> 880 us, FPUT
+// 128 x 512 (w = 1.7) 650 -> 607, 64 x 600 (w = 1) 354 -> 487).
+bool mixed_few_sites(const nlc_plan &P, int model, const RealShape &s) {
+	const double w = double(P.m.copies) * s.lanes / (128. * P.prop.multiProcessorCount);
+	return model == NLC_TODA ? w >= 0.5 : w >= 1.5 && w * s.sites >= 3.;
+}
+
 // Canonical: the smallest group whose lanes hold at most 8 sites, from the chain length alone.
 RealShape canonical_shape(const nlc_plan &P, int model, int variant) {
 	for (auto c : shape_candidates(P.m.chain_length)) {
@@ -416,6 +428,7 @@ RealShape autotune_shape(nlc_plan &P, int model, int variant) {
 		const int tpb = cand.second;
 		if (!finish_shape(P, model, variant, s, tpb)) continue;
 		if (s.lanes <= 32 && s.threads != std::max(tpb, s.lanes)) continue;
+		a.mixed = mixed_few_sites(P, model, s);
 		float ms = 1e30f;
 		bool ok = true;
 		for (int rep = 0; rep < 4 && ok; rep++) {
@@ -1096,7 +1109,7 @@ extern "C" int nlc_plan_create(const nlc_model *model, nlc_plan **out) {
 			P->rs.blocks = int(std::min<unsigned long long>((model->copies + gpb - 1) / gpb, 0x7fffffffull));
 		}
 		a.lanes = P->rs.lanes;
-		a.mixed = (unsigned long long) model->copies * P->rs.lanes >= 64ull * P->prop.multiProcessorCount;
+		a.mixed = mixed_few_sites(*P, mdl, P->rs);
 		P->tier = P->win_len ? 4 : P->rs.lanes > 32 ? 2 : 1;
 		int per_sm = 1;
 		cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, real_move_kernel(mdl, P->variant, P->rs.sites, P->win_len != 0),

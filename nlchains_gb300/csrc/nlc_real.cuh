@@ -34,6 +34,7 @@
 //   Toda 13 (12 with 2 alpha == 1) including the 8-operation table exp: the two subtractions, the index,
 //     its value and half the polynomial of the exp, 6 left.  N = 128, 16384 chains, 100 steps: 32.9 ->
 //     17.2 ms (20.1 with the index and the polynomial's sum still on the FP64 pipe).
+// Lanes of up to 3 sites use both where that is faster (mixed_few_sites in nlc_plan.cpp).
 #pragma once
 
 #include <type_traits>
@@ -48,24 +49,32 @@ namespace nlc {
 // one warp (width-G shuffles); otherwise warp-boundary halos go through shared memory.  The kernel
 // picks the form once per launch, outside the step loop, so that for SHFL the seven sub-steps of a
 // step are one straight-line block the compiler can schedule across.
+// FEW: lanes of up to 3 sites, whose sub-steps are short enough for the other warps' indices to matter
+// (kept in a register; FPUT N = 64, 1024 chains 492 us for 100 steps, 581 worked out at each use); with
+// more sites the register is worth more (Toda N = 128, 16384 chains 17.06 ms, 17.46 with it kept).  By masks, as
+// the warps per chain are a power of two: a remainder at each exchange took 90 instructions.
+template <bool FEW>
 struct Ring {
 	int G;          // lanes per chain
 	int lane;       // lane index within the chain
 	int wl;         // lane index within the warp
 	int warp;       // warp index within the block (G > 32 only)
-	int W;          // warps per chain (G > 32 only)
-	double *xbuf;   // 2 parities x 2 directions x W doubles (G > 32 only)
+	double *xbuf;   // 2 parities x 2 directions x W doubles, W the warps per chain (G > 32 only)
 	int parity;
+	int kept_W;     // FEW: W
+
+	__device__ __forceinline__ int warps() const { return FEW ? kept_W : G >> 5; }
 
 	// value of lane (lane - 1) mod G
 	template <bool SHFL>
 	__device__ __forceinline__ double from_left(double v) {
 		if constexpr (SHFL) return __shfl_sync(0xffffffffu, v, (lane + G - 1) & (G - 1), G);
 		double a = __shfl_sync(0xffffffffu, v, (wl + 31) & 31);
+		const int W = warps();
 		double *buf = xbuf + parity * 2 * W;
 		if (wl == 31) buf[warp] = v;
 		__syncthreads();
-		if (wl == 0) a = buf[(warp + W - 1) % W];
+		if (wl == 0) a = buf[(warp + W - 1) & (W - 1)];
 		parity ^= 1;
 		return a;
 	}
@@ -75,10 +84,11 @@ struct Ring {
 	__device__ __forceinline__ double from_right(double v) {
 		if constexpr (SHFL) return __shfl_sync(0xffffffffu, v, (lane + 1) & (G - 1), G);
 		double a = __shfl_sync(0xffffffffu, v, (wl + 1) & 31);
+		const int W = warps();
 		double *buf = xbuf + parity * 2 * W + W;
 		if (wl == 0) buf[warp] = v;
 		__syncthreads();
-		if (wl == 31) a = buf[(warp + 1) % W];
+		if (wl == 31) a = buf[(warp + 1) & (W - 1)];
 		parity ^= 1;
 		return a;
 	}
@@ -93,12 +103,13 @@ struct Ring {
 		}
 		left = __shfl_sync(0xffffffffu, to_right, (wl + 31) & 31);
 		right = __shfl_sync(0xffffffffu, to_left, (wl + 1) & 31);
+		const int W = warps();
 		double *buf = xbuf + parity * 2 * W;
 		if (wl == 31) buf[warp] = to_right;
 		if (wl == 0) buf[W + warp] = to_left;
 		__syncthreads();
-		if (wl == 0) left = buf[(warp + W - 1) % W];
-		if (wl == 31) right = buf[W + (warp + 1) % W];
+		if (wl == 0) left = buf[(warp + W - 1) & (W - 1)];
+		if (wl == 31) right = buf[W + ((warp + 1) & (W - 1))];
 		parity ^= 1;
 	}
 };
@@ -132,6 +143,20 @@ __device__ __forceinline__ double bond_force_mixed(double d, const ForceConsts &
 	}
 }
 
+// The operations that a lane of fewer than kInlineRedo sites redoes on the FP64 pipe, as functions of
+// their own: a few FP64 instructions under a branch become predicated ones, which occupy the pipe
+// whether redone or not.
+constexpr int kInlineRedo = 4;
+static __device__ __noinline__ double sub_redo(double a, double b) { return dadd(a, -b); }
+template <int VAR>
+__device__ __noinline__ double fput_redo(double d, double alpha, double beta) {
+	return dmul(d, dfma(VAR ? d : dfma(beta, d, alpha), d, 1.));
+}
+template <int VAR>
+__device__ __noinline__ double on_site_redo(double l, double c, double r, double mp2, double beta) {
+	return dadd(dfma(c, dfma(VAR ? c : dmul(beta, c), c, mp2), -l), -r);
+}
+
 // Integer-pipe operations are checked (and redone) this many sites at a time, so that a batch's
 // operands stay in registers until then.
 constexpr int kIntBatch = 8;
@@ -151,7 +176,8 @@ __device__ __forceinline__ void sub_batch(double *out, const double *a, const do
 			for (int j = j0; j < E && j < j0 + kIntBatch; j++) out[j] = int_sub(a[j], b[j], j == E - 1 ? fe : f);
 			if (__any_sync(0xffffffffu, f.bad() | (last & fe.bad()))) {
 #pragma unroll
-				for (int j = j0; j < E && j < j0 + kIntBatch; j++) out[j] = fsub(a[j], b[j], k);
+				for (int j = j0; j < E && j < j0 + kIntBatch; j++)
+					out[j] = E < kInlineRedo ? sub_redo(a[j], b[j]) : fsub(a[j], b[j], k);
 			}
 		}
 	}
@@ -178,7 +204,7 @@ __global__ void __launch_bounds__(kMaxThreads<MODEL, E, WIN>) real_move_kernel_t
 	const int gib = tid / G;                 // group (chain) in block
 	const int gpb = blockDim.x / G;          // groups per block
 
-	Ring ring{G, lane, tid & 31, tid >> 5, G > 32 ? G >> 5 : 1, xbuf, 0};
+	Ring<(E < kInlineRedo)> ring{G, lane, tid & 31, tid >> 5, xbuf, 0, G > 32 ? G >> 5 : 1};
 
 	// the constants and, per sub-step, the coefficients as vector-register operands (nlc_device.cuh)
 	const int zero = lane_zero(a.k1);
@@ -294,7 +320,7 @@ __global__ void __launch_bounds__(kMaxThreads<MODEL, E, WIN>) real_move_kernel_t
 				for (int j = 0; j < E; j++) x[j + 1] = dfma(a.cd_final, p[j], x[j + 1]);
 			}
 			rpos++;
-#pragma unroll (INT ? 1 : 7)
+#pragma unroll (INT && E >= 4 ? 1 : 7)
 			for (int k = 0; k < 7; k++) {
 				// the trailing drift of step i-1 (c[7]) merged with the leading drift of step i (c[0])
 				const double cd = in_register(k == 0 ? (i == 0 ? cd_lead : boundary ? a.cd[0] : a.cd0_merged) : a.cd[k], zero);
@@ -345,7 +371,9 @@ __global__ void __launch_bounds__(kMaxThreads<MODEL, E, WIN>) real_move_kernel_t
 								}
 								if (__any_sync(0xffffffffu, mv_bad | f.bad() | (fl & fe.bad()))) {
 #pragma unroll
-									for (int j = j0; j <= E && j < j0 + kIntBatch; j++) v[j - j0] = force_fp64(j);
+									for (int j = j0; j <= E && j < j0 + kIntBatch; j++)
+										v[j - j0] = E < kInlineRedo ? on_site_redo<VAR>(x[j - 1], x[j], x[j + 1], mp2(j), fc.beta)
+										                            : force_fp64(j);
 								}
 #pragma unroll
 								for (int j = j0; j <= E && j < j0 + kIntBatch; j++) p[j - 1] = dfma(ck, v[j - j0], p[j - 1]);
@@ -373,8 +401,12 @@ __global__ void __launch_bounds__(kMaxThreads<MODEL, E, WIN>) real_move_kernel_t
 							}
 							if (__any_sync(0xffffffffu, f.bad() | (fl & fe.bad()))) {
 #pragma unroll
-								for (int j = j0; j <= E && j < j0 + kIntBatch; j++)
-									g[j] = bond_force<MODEL, VAR>(fsub(x[j + 1], x[j], k1), fc, k1, s_tab);
+								for (int j = j0; j <= E && j < j0 + kIntBatch; j++) {
+									if constexpr (MODEL == NLC_FPUT && E < kInlineRedo)
+										g[j] = fput_redo<VAR>(sub_redo(x[j + 1], x[j]), fc.alpha, fc.beta);
+									else
+										g[j] = bond_force<MODEL, VAR>(fsub(x[j + 1], x[j], k1), fc, k1, s_tab);
+								}
 							}
 						}
 					}
@@ -387,19 +419,16 @@ __global__ void __launch_bounds__(kMaxThreads<MODEL, E, WIN>) real_move_kernel_t
 			}
 		}
 		};
-		// Operations on the integer pipes from 4 sites per lane on.  Lanes of fewer sites are those of
-		// ensembles too small to fill the schedulers, or of short chains: with a warp or two per scheduler
-		// the two pipes hardly overlap (a warp issues in order) and an operation costs 75 clocks against 64
-		// (FPUT N = 64, 100 steps, one site per lane: 232 us for 96 chains with the FP64 pipe alone, 403 with
-		// both; 1024 chains 497 against 679).  Toda, with 12 operations a site, gains from two warps
-		// per SM on (a.mixed; N = 128, 512 chains: 1082 -> 958 us; N = 64, 96 chains: 419 against 560).
+		// Operations on the integer pipes from 4 sites per lane on, and with fewer where there are warps
+		// enough for the two pipes to overlap (a.mixed): lanes of few sites are those of ensembles too small
+		// to fill the schedulers, or of short chains
 		if constexpr (E >= 4) {
 			if (G <= 32) integrate(std::true_type{}, std::true_type{});
 			else integrate(std::false_type{}, std::true_type{});
 		} else {
-			if (MODEL == NLC_TODA && a.mixed) {
-				if (G <= 32) integrate(std::true_type{}, std::bool_constant<MODEL == NLC_TODA>{});
-				else integrate(std::false_type{}, std::bool_constant<MODEL == NLC_TODA>{});
+			if (a.mixed) {
+				if (G <= 32) integrate(std::true_type{}, std::true_type{});
+				else integrate(std::false_type{}, std::true_type{});
 			} else {
 				if (G <= 32) integrate(std::true_type{}, std::false_type{});
 				else integrate(std::false_type{}, std::false_type{});

@@ -70,6 +70,32 @@ def test_bits_at_edge_operands(gpu, monkeypatch, model, params, n, lanes):
     assert not bad.any(), f"rows {np.unique(np.nonzero(bad)[0])}: {np.count_nonzero(bad)} values differ"
 
 
+# lanes of one, two and three sites take the integer pipes too from a few warps per scheduler on: the same
+# chains, many times over
+@pytest.mark.parametrize("n,lanes", [(16, 16), (64, 64), (5, 4), (200, 128), (23, 8)])
+@pytest.mark.parametrize("model,params", MODELS, ids=lambda v: v if isinstance(v, str) else "-".join(map(str, v.values())))
+def test_bits_of_few_sites_per_lane_in_large_ensembles(gpu, monkeypatch, model, params, n, lanes):
+    monkeypatch.setenv("NLC_FORCE_LANES", str(lanes))
+    masses = ic.masses_uniform(n, seed=n) if model == "dDNKG" else None
+    rows = edge_states(n, n)
+    reps = -(-4 * 128 * 160 // (lanes * len(rows)))   # over 4 warps for each of 160 x 4 schedulers
+    copies = reps * len(rows)
+    ctx = gpu.Context(0)
+    job = ctx.job(gpu.Model(model, n, copies, 0.05, masses=masses, **params), 4)
+    job.upload(np.tile(rows, (reps, 1, 1)))
+    job.advance(4)
+    out = job.download().reshape(reps, len(rows), n, 2)
+    job.close()
+    ctx.close()
+    exp = O.advance(O.Model(model, n, len(rows), 0.05, masses=masses, **params), rows, 4, 4, order=O.ORDER_DEVICE)
+    exp = exp.reshape(len(rows), n, 2)
+    finite = np.isfinite(exp)
+    for r in (0, reps // 2, reps - 1):
+        assert np.array_equal(finite, np.isfinite(out[r]))
+        bad = (out[r].view(np.uint64) != exp.view(np.uint64)) & finite
+        assert not bad.any(), f"rows {np.unique(np.nonzero(bad)[0])}: {np.count_nonzero(bad)} values differ"
+
+
 # sites per lane 1 .. 16 (rows over several chains of a warp, one chain of a warp, a block), every radius, and
 # windows
 @pytest.mark.parametrize("n,dt,sites,window", [(16, 0.01, 0, 0), (33, 0.01, 1, 0), (64, 0.01, 2, 0), (24, 0.05, 12, 0),
