@@ -601,9 +601,12 @@ int setup_tc_projection(nlc_plan &P, const double *d_omega, int slices) {
 	const size_t sms = size_t(P.prop.multiProcessorCount), tiles = tc_projection_tiles(t), rest = tiles % sms;
 	t.parts = rest ? int(std::min<size_t>((t.kp + 255) / 256, sms / rest)) : 1;
 	t.whole = int(t.parts > 1 ? tiles - rest : tiles);
+	if (t.parts > 1 && P.dalloc(&t.part_sums, rest * t.parts * 128 * 128)) {
+		cudaGetLastError();
+		t.parts = 1, t.whole = int(tiles);   // no memory for the parts' sums
+	}
 	if (t.parts > 1) {
 		const std::vector<unsigned int> zero(2 * rest, 0);
-		if ((rc = P.dalloc(&t.part_sums, rest * t.parts * 128 * 128))) return rc;
 		if ((rc = P.upload(&t.part_count, zero.data(), zero.size()))) return rc;
 		t.part_fail = reinterpret_cast<int *>(t.part_count + rest);
 	}
@@ -1085,6 +1088,7 @@ extern "C" int nlc_plan_create(const nlc_model *model, nlc_plan **out) {
 		// NLC_FORCE_WINDOW=<G> integrates in windows of G lanes even where one block holds the chain
 		// (used by the tests to cover the windowed tier on short chains)
 		const char *force_win = std::getenv("NLC_FORCE_WINDOW");
+		RealShape block{};   // the shape to go back to without memory for the windows' second buffer
 		if (force_win) P->rs = RealShape{};
 		// Chains on one block of 256 lanes or more also run in windows where those are estimated faster (few
 		// chains, or blocks too large to run two to an SM: DNKG n = 7000, 200 chains, 50 steps 4.88 ms on
@@ -1092,7 +1096,8 @@ extern "C" int nlc_plan_create(const nlc_model *model, nlc_plan **out) {
 		else if (P->rs.lanes >= 256 && !std::getenv("NLC_FORCE_LANES") && !(model->flags & NLC_FLAG_CANONICAL_SHAPE)) {
 			double cost = 0;
 			const RealShape w = window_shape(*P, mdl, P->variant, 0, &cost);
-			if (w.blocks && cost < 0.95 * block_tier_cost(*P, mdl, P->variant, P->rs, false, model->copies)) P->rs = RealShape{};
+			if (w.blocks && cost < 0.95 * block_tier_cost(*P, mdl, P->variant, P->rs, false, model->copies))
+				block = P->rs, P->rs = RealShape{};
 		}
 		if (!P->rs.blocks) {
 			// longer than one block's registers hold, or faster so: windows of the chain, ping-ponging
@@ -1101,7 +1106,11 @@ extern "C" int nlc_plan_create(const nlc_model *model, nlc_plan **out) {
 			if (!P->rs.blocks) return set_error(NLC_EUNSUPPORTED, "no launchable integrator shape for this chain_length");
 			P->win_len = uint32_t(P->rs.lanes) * P->rs.sites;
 			P->win_steps = std::max<uint32_t>(1, P->win_len / 140);   // discarded ends: 5% of a window each
-			if ((rc = P->dalloc(&P->d_win, size_t(model->copies) * n))) return rc;
+			if ((rc = P->dalloc(&P->d_win, size_t(model->copies) * n))) {
+				if (!block.blocks) return rc;
+				cudaGetLastError();
+				P->rs = block, P->win_len = 0;
+			}
 			P->rs.blocks = std::max(1, P->rs.blocks);
 		}
 		if (model->flags & NLC_FLAG_SHARED_GPU) {
