@@ -645,7 +645,10 @@ int setup_diagnostics(nlc_plan &P) {
 		P.diag_smem = size_t(8) * g.proj_chunk * sizeof(double2);
 		P.diag_team_block = 1;
 		const unsigned long long tiles = (P.m.copies + 7) / 8;
-		P.diag_blocks = int(std::min<unsigned long long>(tiles, 2ull * sms));
+		// 16 warps an SM, four for each scheduler: a block has a warp for every 32 modes (30 sites x 21758
+		// chains 203 -> 105 us a sample against two blocks an SM, 64 x 65536 1108 -> 965)
+		const unsigned per_sm = P.m.flags & NLC_FLAG_COMPACT_DIAG ? 2 : std::max(2, 512 / P.diag_threads);
+		P.diag_blocks = int(std::min<unsigned long long>(tiles, (unsigned long long) per_sm * sms));
 		P.diag_rows = P.diag_blocks;
 		// the tensor-core projection is faster from ~128 sites on (3x at 256, 6x at 1024 sites on GB300)
 		const bool bf16x3 = P.m.flags & NLC_FLAG_BF16X3_PROJECTION;
