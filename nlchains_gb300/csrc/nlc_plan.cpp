@@ -456,16 +456,17 @@ RealShape autotune_shape(nlc_plan &P, int model, int variant) {
 	return best;
 }
 
-// FP64 lane operations of one step of one block of chains_per_block chains, divided by the fraction
-// of the FP64 peak the kernel sustains (an FMA is one operation).  Work per site and step (7
-// sub-steps): the real models' drift, neighbour terms and kick, the Toda exponential (~22
-// operations), the DNLS phase rotation (sincos ~31) and two Stockham transforms (~3 operations per
-// element and radix-2 level).  The request server turns it into a block lifetime to split long rounds.
+// Operations of one step of one block of chains_per_block chains, divided by the multiple of the FP64
+// rate that the kernel does them at.  Work per site and step (7 sub-steps): the real models' 5 to 12
+// operations a sub-step, about half of them beside the FP64 pipe (28.2, 24.6, 16.2 and 12.3 G site-steps/s
+// for large DNKG, dDNKG, FPUT and Toda ensembles); the DNLS phase rotation and two Stockham transforms
+// (~3 operations per element and radix-2 level).  The request server turns it into a block lifetime to
+// split long rounds.
 double block_step_ops(int model, uint32_t n, uint32_t len, bool bluestein, int chains_per_block) {
 	double per_site, eff;
 	switch (model) {
-		case NLC_TODA: per_site = 7 * 32.; eff = 0.8; break;
-		case NLC_FPUT: per_site = 7 * 8.; eff = 0.85; break;
+		case NLC_TODA: per_site = 7 * 12.; eff = 1.7; break;
+		case NLC_FPUT: per_site = 7 * 7.; eff = 1.3; break;
 		case NLC_DNLS: {
 			// a linear sub-step: two passes of n, or with a large prime factor two passes of the
 			// padded convolution length plus its product
@@ -475,7 +476,8 @@ double block_step_ops(int model, uint32_t n, uint32_t len, bool bluestein, int c
 			eff = 0.4;
 			break;
 		}
-		default: per_site = 7 * 6.; eff = 0.85;
+		case NLC_DDNKG: per_site = 7 * 5.; eff = 1.4; break;
+		default: per_site = 7 * 5.; eff = 1.6;
 	}
 	return per_site * double(n) * chains_per_block / eff;
 }
