@@ -54,8 +54,11 @@ __device__ __forceinline__ void add_team_rows(const DiagArgs &a, const double *r
 	}
 }
 
-template <bool BLOCK>
-__global__ void __launch_bounds__(BLOCK ? 512 : 128) lin_fft_kernel(const double2 *__restrict__ state, const DiagArgs a) {
+// GLOBAL: the buffers in global memory, where two blocks of 512 threads an SM hide its latency: 64
+// registers a thread, so no integer-pipe operations (one block at 126 registers against two: 19328 x 403
+// 3486 -> 3257 us, 16384 x 310 652 -> 603).
+template <bool BLOCK, bool GLOBAL = false>
+__global__ void __launch_bounds__(BLOCK ? 512 : 128, GLOBAL ? 2 : 1) lin_fft_kernel(const double2 *__restrict__ state, const DiagArgs a) {
 	extern __shared__ double2 sm[];
 	const int n = int(a.n);
 	const int T = BLOCK ? blockDim.x : 32;
@@ -63,7 +66,7 @@ __global__ void __launch_bounds__(BLOCK ? 512 : 128) lin_fft_kernel(const double
 	const int team = BLOCK ? 0 : (threadIdx.x >> 5);
 	const int teams = BLOCK ? 1 : (blockDim.x >> 5);
 	const int len = a.fft.len;
-	double2 *x = BLOCK && a.gscratch ? a.gscratch + (size_t) blockIdx.x * 2 * len : sm + (size_t) team * 2 * len;
+	double2 *x = GLOBAL ? a.gscratch + (size_t) blockIdx.x * 2 * len : sm + (size_t) team * 2 * len;
 	double2 *y = x + len;
 	double *const rows = reinterpret_cast<double *>(sm + (size_t) teams * 2 * len);
 	double *const acc = team_row<BLOCK>(a, rows, team, t, T);
@@ -75,13 +78,13 @@ __global__ void __launch_bounds__(BLOCK ? 512 : 128) lin_fft_kernel(const double
 		const double2 *src = state + chain * (unsigned long long) n;
 		for (int k = t; k < n; k += T) x[k] = src[k];
 		team_sync<BLOCK>();
-		const double2 *Z = fft_team<BLOCK, false>(a.fft, k1, x, y, t, T);
+		const double2 *Z = fft_team<BLOCK, false, !GLOBAL>(a.fft, k1, x, y, t, T);
 		if (dnls) {
 			for (int k = t; k < n; k += T) {
 				const double2 z = Z[k];
 				IntFlags f;
 				double e;
-				if (a.mixed) {
+				if (!GLOBAL && a.mixed) {
 					e = dfma(z.x, z.x, int_mul(z.y, z.y, f));
 					if (any_bad(f)) e = norm_fp64(z);
 				} else {
@@ -95,7 +98,7 @@ __global__ void __launch_bounds__(BLOCK ? 512 : 128) lin_fft_kernel(const double
 				const double ak = a.coef_a[k], bk = a.coef_b[k];
 				IntFlags f;
 				double e;
-				if (a.mixed) {
+				if (!GLOBAL && a.mixed) {
 					const double re = dfma(ak, zk.x, int_mul(bk, zm.x, f));
 					const double im = dfma(ak, zk.y, -int_mul(bk, zm.y, f));
 					e = dfma(re, re, int_mul(im, im, f));
@@ -347,6 +350,8 @@ cudaError_t launch_linenergies_partials(const DiagArgs &a, const void *state, in
 	} else if (a.tw32) {
 		if (team_block) lin_fft32_kernel<true><<<blocks, threads, smem / 2, stream>>>(st, a);
 		else lin_fft32_kernel<false><<<blocks, threads, smem / 2 + rows, stream>>>(st, a);
+	} else if (a.gscratch) {
+		lin_fft_kernel<true, true><<<blocks, threads, smem, stream>>>(st, a);
 	} else if (team_block) {
 		lin_fft_kernel<true><<<blocks, threads, smem, stream>>>(st, a);
 	} else {
@@ -362,7 +367,7 @@ cudaError_t launch_linenergies_partials(const DiagArgs &a, const void *state, in
 // counter, no waiting) adds those of all blocks in a fixed order.  The result is identical on every run.
 // What it costs is latency: the launches, the loads' round trips and the serial sums.  One launch with
 // eight loads in flight per thread and a row per block, against one launch for slices of the rows and
-// one or two to finish them over a row per team: a sample of 64 sites x 96 copies in a job with 100
+// one or two to finish them over a row per team: a sample of 64 sites x 96 copies in a job with 10
 // steps 71.1 -> 66.7 us in all, 128 x 65536 336 -> 328 us, 512 x 64 48.6 -> 22.6 us, 4096 x 512
 // 221 -> 195 us.  Four to eight blocks of 1024 threads over a row per team instead take 9 us more than
 // those launches at 128 x 65536: a few SMs cannot draw 2 MB from L2 in that time.

@@ -83,7 +83,7 @@ struct NoMap {
 // pass applies `pre` to its inputs (the first pass) / `post` to its outputs (the last pass); they
 // are template flags so that the other passes carry no trace of the maps.  k: the FP64 constants in
 // vector registers (nlc_device.cuh).
-template <bool BLOCK, bool INV, bool PRE, bool POST, class Pre, class Post>
+template <bool BLOCK, bool INV, bool INT, bool PRE, bool POST, class Pre, class Post>
 __device__ __forceinline__ void stockham_pass(const FftPlanDev &P, const FpOnes &k, int r, int Ns, double2 *x, double2 *y,
                                               int t, int T, const Pre &pre, const Post &post) {
 	const int n = P.len;
@@ -133,10 +133,11 @@ __device__ __forceinline__ void stockham_pass(const FftPlanDev &P, const FpOnes 
 					X0 = add(b0, b2), X1 = add(b1, b3), X2 = sub(b0, b2), X3 = sub(b1, b3);
 				};
 				IntFlags f;
-				if (!P.fp64_first)
+				const bool fp64 = !INT || P.fp64_first;
+				if (!fp64)
 					butterfly([&](double2 u, double2 v) { return make_double2(int_add(u.x, v.x, f), int_add(u.y, v.y, f)); },
 					          [&](double2 u, double2 v) { return make_double2(int_sub(u.x, v.x, f), int_sub(u.y, v.y, f)); });
-				if (P.fp64_first || any_bad(f))
+				if (fp64 || any_bad(f))
 					butterfly([&](double2 u, double2 v) { return cadd(u, v, k); }, [&](double2 u, double2 v) { return csub(u, v, k); });
 				store4(4 * b, b, X0, X1, X2, X3);
 			}
@@ -241,41 +242,42 @@ __device__ __forceinline__ void stockham_pass(const FftPlanDev &P, const FpOnes 
 		}
 	} else {
 		// direct p-point DFT of the twiddled inputs: X_v = sum_u a_u w^{uk} W_p^{uv}
-		// = sum_u a_u tw[u (k + v Ns) n / (Ns p) mod n]
+		// = sum_u a_u tw[u (k + v Ns) n / (Ns p) mod n].  A thread per output, not per butterfly: a pass of a
+		// large prime has few butterflies (644 = 4 x 7 x 23: 28), whose p^2 products would be one thread's
+		// (energies of 38 = 2 x 19 sites x 20000 chains 1597 -> 205 us, 644 x 60 145 -> 43, 1690 x 856 480 -> 388).
 		const int stride = n / (Ns * p);
-		for (int b = t; b < m; b += T) {
+		for (int i = t; i < n; i += T) {
+			const int v = i / m, b = i - v * m;
 			const int q = b / Ns, kk = b - q * Ns;
-			for (int v = 0; v < p; v++) {
-				const int step = int((long long) (kk + v * Ns) * stride % n);
-				double re = 0., im = 0.;
-				int e = 0;
-				for (int u = 0; u < p; u++) {
-					const double2 a = x[b + u * m];
-					const double2 w = twiddle<INV>(tw, e);
-					re = dfma(a.x, w.x, dfma(-a.y, w.y, re));
-					im = dfma(a.x, w.y, dfma(a.y, w.x, im));
-					e += step;
-					if (e >= n) e -= n;
-				}
-				out(q * p * Ns + kk, v, make_double2(re, im));
+			const int step = (kk + v * Ns) * stride;   // below n
+			double re = 0., im = 0.;
+			int e = 0;
+			for (int u = 0; u < p; u++) {
+				const double2 a = x[b + u * m];
+				const double2 w = twiddle<INV>(tw, e);
+				re = dfma(a.x, w.x, dfma(-a.y, w.y, re));
+				im = dfma(a.x, w.y, dfma(a.y, w.x, im));
+				e += step;
+				if (e >= n) e -= n;
 			}
+			out(q * p * Ns + kk, v, make_double2(re, im));
 		}
 	}
 }
 
 // Stockham transform of length P.len on x (shared memory), y the ping-pong buffer.  t / T: this
 // thread's index / size of the team.  Returns the buffer holding the result.
-template <bool BLOCK, bool INV, class Pre = NoMap, class Post = NoMap>
+template <bool BLOCK, bool INV, bool INT = true, class Pre = NoMap, class Post = NoMap>
 __device__ double2 *stockham_team(const FftPlanDev &P, const FpOnes &k, double2 *x, double2 *y, int t, int T, Pre pre = Pre(),
                                   Post post = Post()) {
 	constexpr bool kPre = !std::is_same<Pre, NoMap>::value, kPost = !std::is_same<Post, NoMap>::value;
 	int Ns = 1;
 	for (int r = 0; r < P.nradix; r++) {
 		const bool first = r == 0, last = r == P.nradix - 1;
-		if (kPre && kPost && first && last) stockham_pass<BLOCK, INV, kPre, kPost>(P, k, r, Ns, x, y, t, T, pre, post);
-		else if (kPre && first) stockham_pass<BLOCK, INV, kPre, false>(P, k, r, Ns, x, y, t, T, pre, post);
-		else if (kPost && last) stockham_pass<BLOCK, INV, false, kPost>(P, k, r, Ns, x, y, t, T, pre, post);
-		else stockham_pass<BLOCK, INV, false, false>(P, k, r, Ns, x, y, t, T, pre, post);
+		if (kPre && kPost && first && last) stockham_pass<BLOCK, INV, INT, kPre, kPost>(P, k, r, Ns, x, y, t, T, pre, post);
+		else if (kPre && first) stockham_pass<BLOCK, INV, INT, kPre, false>(P, k, r, Ns, x, y, t, T, pre, post);
+		else if (kPost && last) stockham_pass<BLOCK, INV, INT, false, kPost>(P, k, r, Ns, x, y, t, T, pre, post);
+		else stockham_pass<BLOCK, INV, INT, false, false>(P, k, r, Ns, x, y, t, T, pre, post);
 		team_sync<BLOCK>();
 		double2 *sw = x;
 		x = y, y = sw;
@@ -327,22 +329,22 @@ __device__ float2 *stockham32_team(const FftPlanDev &P, const float2 *__restrict
 				o[Ns] = make_float2(a0.x - a1.x, a0.y - a1.y);
 			}
 		} else {
-			// direct p-point DFT of the twiddled inputs: X_v = sum_u a_u tw[u (k + v Ns) stride mod n]
-			for (int b = t; b < m; b += T) {
+			// direct p-point DFT of the twiddled inputs: X_v = sum_u a_u tw[u (k + v Ns) stride mod n], a
+			// thread per output
+			for (int i = t; i < n; i += T) {
+				const int v = i / m, b = i - v * m;
 				const int q = b / Ns, kk = b - q * Ns;
-				for (int v = 0; v < p; v++) {
-					const int step = int((long long) (kk + v * Ns) * stride % n);
-					float re = 0.f, im = 0.f;
-					int e = 0;
-					for (int u = 0; u < p; u++) {
-						const float2 a = x[b + u * m], w = tw[e];
-						re = fmaf(a.x, w.x, fmaf(-a.y, w.y, re));
-						im = fmaf(a.x, w.y, fmaf(a.y, w.x, im));
-						e += step;
-						if (e >= n) e -= n;
-					}
-					y[q * p * Ns + kk + v * Ns] = make_float2(re, im);
+				const int step = (kk + v * Ns) * stride;   // below n
+				float re = 0.f, im = 0.f;
+				int e = 0;
+				for (int u = 0; u < p; u++) {
+					const float2 a = x[b + u * m], w = tw[e];
+					re = fmaf(a.x, w.x, fmaf(-a.y, w.y, re));
+					im = fmaf(a.x, w.y, fmaf(a.y, w.x, im));
+					e += step;
+					if (e >= n) e -= n;
 				}
+				y[q * p * Ns + kk + v * Ns] = make_float2(re, im);
 			}
 		}
 		team_sync<BLOCK>();
@@ -362,9 +364,9 @@ __device__ __forceinline__ double2 conj2(double2 a) { return make_double2(a.x, -
 // (L. Bluestein, IEEE Trans. Audio Electroacoust. 18, 1970), the convolution evaluated as a cyclic
 // convolution of smooth length m >= 2n - 1 by two Stockham passes; the backward transform uses the
 // conjugate chirp.  Returns the buffer holding X[0, n).
-template <bool BLOCK, bool INV>
+template <bool BLOCK, bool INV, bool INT = true>
 __device__ double2 *fft_team(const FftPlanDev &P, const FpOnes &k, double2 *x, double2 *y, int t, int T) {
-	if (!P.bluestein) return stockham_team<BLOCK, INV>(P, k, x, y, t, T);
+	if (!P.bluestein) return stockham_team<BLOCK, INV, INT>(P, k, x, y, t, T);
 	const int n = P.n, m = P.len;
 	for (int j = t; j < m; j += T) {
 		if (j < n) {
@@ -375,12 +377,12 @@ __device__ double2 *fft_team(const FftPlanDev &P, const FpOnes &k, double2 *x, d
 		}
 	}
 	team_sync<BLOCK>();
-	double2 *r = stockham_team<BLOCK, false>(P, k, y, x, t, T);
+	double2 *r = stockham_team<BLOCK, false, INT>(P, k, y, x, t, T);
 	double2 *o = r == y ? x : y;
 	const double2 *__restrict__ b = INV ? P.bi : P.bf;
 	for (int j = t; j < m; j += T) r[j] = cmul(r[j], b[j], k);
 	team_sync<BLOCK>();
-	double2 *c = stockham_team<BLOCK, true>(P, k, r, o, t, T);
+	double2 *c = stockham_team<BLOCK, true, INT>(P, k, r, o, t, T);
 	for (int j = t; j < n; j += T) {
 		const double2 w = P.chirp[j];
 		c[j] = cmul(c[j], INV ? conj2(w) : w, k);

@@ -699,8 +699,8 @@ int setup_diagnostics(nlc_plan &P) {
 			while (T < 512 && uint32_t(T) * 4 < len && (unsigned long long) P.m.copies * T < 256ull * sms) T <<= 1;
 			P.diag_threads = T;
 			P.diag_smem = size_t(2) * len * sizeof(double2);
-			// resident blocks, in shared memory and (at 125 registers) in the register file
-			int per_sm = int(std::min<size_t>(P.prop.sharedMemPerMultiprocessor / (P.diag_smem + 1024), size_t(512 / T)));
+			// resident blocks, in shared memory and (at 96 registers) in the register file
+			int per_sm = int(std::min<size_t>(P.prop.sharedMemPerMultiprocessor / (P.diag_smem + 1024), size_t(640 / T)));
 			per_sm = std::max(per_sm, 2);
 			if (compact) per_sm = len <= 1024 ? 2 : 1;
 			P.diag_blocks = int(std::min<unsigned long long>(P.m.copies, (unsigned long long) per_sm * sms));
@@ -712,7 +712,7 @@ int setup_diagnostics(nlc_plan &P) {
 				if ((rc = P.dalloc(&g.gscratch, size_t(P.diag_blocks) * 2 * len))) return rc;
 			}
 		}
-		g.mixed = (unsigned long long) P.diag_blocks * (P.diag_threads / 32) >= 8ull * sms;
+		g.mixed = !g.gscratch && (unsigned long long) P.diag_blocks * (P.diag_threads / 32) >= 8ull * sms;
 		if (!g.mixed) g.fft.fp64_first = 1;
 		// FP32 diagnostics: for direct transforms held in shared memory (padded lengths and
 		// global-memory passes keep the FP64 transform)

@@ -155,3 +155,14 @@ def test_ddnkg_device_eigensystem_equals_host(gpu, n, monkeypatch):
         plan.close()
     assert np.abs(out[False][0] - out[True][0]).max() <= 1e-12 * out[True][0].max()
     assert np.abs(out[False][1] - out[True][1]).max() <= 1e-10 * np.abs(out[True][1]).max()
+
+
+# direct passes of a prime (fewer butterflies than a team's threads, and more) in warp teams and blocks;
+# transforms in global memory, direct and padded
+@pytest.mark.parametrize("n,copies", [(38, 700), (253, 61), (644, 40), (1690, 21), (2197, 9), (7488, 5), (7753, 3)])
+def test_prime_passes_and_global_memory(gpu, n, copies):
+    state = np.random.default_rng(n).standard_normal((copies, n, 2))
+    params = dict(m=1.0, beta=1.0)
+    lin, wt, inf = diag(gpu, "DNKG", n, copies, params, state)
+    mdl = O.Model("DNKG", n, copies, 0.05, **params)
+    check(lin, wt, inf, O.linenergies(mdl, state), O.a0is0(mdl))
