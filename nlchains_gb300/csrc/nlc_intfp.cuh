@@ -177,8 +177,10 @@ __device__ __forceinline__ int int_exp_index(double x, const ExpConsts &c, IntFl
 	return (n ^ neg) - neg;
 }
 
-// 1 + a b, |a b| < 1/4 (flagged): the exact product's top 64 bits shifted to the scale of 2^-62, the rest
-// ORed into the lowest one, added to or subtracted from 2^62; the sum's leading bit is at 62 or 61.
+// 1 + a b, |a b| < 1/2 (flagged): the exact product's top 64 bits shifted to the scale of 2^-62, the rest
+// ORed into the lowest one, added to or subtracted from 2^62; the sum's leading bit is at 62 or 61.  The
+// product is that of two significands, below 4, times 2^-t: below 1/2 from t = 3 on.  a is of an ordinary
+// size (the caller's: a polynomial near 1/2), b any double.
 __device__ __forceinline__ double int_one_plus(double a, double b, IntFlags &f) {
 	const uint32_t ah = __double2hiint(a), a0 = __double2loint(a), bh = __double2hiint(b), b0 = __double2loint(b);
 	const uint32_t a1 = (ah & 0xfffffu) | 0x100000u, b1 = (bh & 0xfffffu) | 0x100000u;
@@ -201,7 +203,7 @@ __device__ __forceinline__ double int_one_plus(double a, double b, IntFlags &f) 
 	const uint32_t drop = 10u - z, half = ((rl >> drop) & 1u) + (0x200u >> z) - 1u;
 	uint32_t ol, oh;
 	asm("{add.cc.u32 %0, %2, %3; addc.u32 %1, %4, 0;}" : "=r"(ol), "=r"(oh) : "r"(rl), "r"(half), "r"(rh));
-	f.rmin = min(f.rmin, t - 1);
+	f.rmin = min(f.rmin, t - 2);
 	return __hiloint2double(int((oh >> drop) + 0x3fe00000u - z * 0x100000u), int(__funnelshift_r(ol, oh, drop)));
 }
 
