@@ -132,7 +132,8 @@ struct nlc_plan {
 	bool tc = false;
 	TcArgs tca{};
 	uint32_t win_len = 0, win_steps = 0;   // windowed tier: sites per window, steps per launch
-	double2 *d_win = nullptr;              // windowed tier: the second state buffer
+	double2 *d_win = nullptr;              // windowed tier: the second state buffer,
+	uint32_t win_copies = 0;               // of as many chains (those of one pass, see window_buffer)
 	double block_ops = 0;      // FP64 work of one block's step over the sustained fraction of peak
 	int per_sm = 1, block_warps = 1;   // resident blocks per SM, warps per block of the move kernel
 	double step_us = 0;        // measured time of one step of the whole ensemble (autotuner), 0 = not timed
@@ -516,6 +517,24 @@ RealShape window_shape(const nlc_plan &P, int model, int variant, int only_lanes
 	return best;
 }
 
+// The second state buffer of the windowed tiers.  An ensemble larger than it is advanced in passes, each
+// of as many chains as it holds through all the steps of a call, so that a plan needs little memory
+// beside the state, also of an ensemble that fills the device.  1 GiB is 64 Mi sites: a pass's launches take
+// milliseconds, its last round of windows under 1% of one; a 32nd of the free memory at most, as
+// the caller's state may be still to come.
+constexpr size_t kWindowBufferBytes = size_t(1) << 30;
+
+int window_buffer(nlc_plan &P) {
+	size_t free_bytes = 0, total = 0;
+	int rc = cuda_status(cudaMemGetInfo(&free_bytes, &total), "cudaMemGetInfo");
+	if (rc) return rc;
+	const size_t chain = size_t(P.m.chain_length) * sizeof(double2);
+	const size_t most = std::max<size_t>(1, std::min(kWindowBufferBytes, free_bytes / 32) / chain);
+	const size_t passes = (P.m.copies + most - 1) / most;
+	P.win_copies = uint32_t((P.m.copies + passes - 1) / passes);
+	return P.dalloc(&P.d_win, P.win_copies * size_t(P.m.chain_length));
+}
+
 // the longest pass length whose two buffers (2 x len complex) fit one block's shared memory
 uint32_t smem_fft_len(const nlc_plan &P) {
 	return uint32_t(P.prop.sharedMemPerBlockOptin / (2 * sizeof(double2))) - 64;
@@ -874,8 +893,7 @@ static int setup_dnls_stencil(nlc_plan &P) {
 	if (windowed) {
 		P.win_len = uint32_t(lanes) * sites;
 		P.win_steps = dnls_window_steps(P.win_len, R);
-		int rc2;
-		if ((rc2 = P.dalloc(&P.d_win, size_t(P.m.copies) * n))) return rc2;
+		if ((rc = window_buffer(P))) return rc;
 		P.dnls_blocks = per_sm * P.prop.multiProcessorCount;   // per launch: at most one block per window
 	}
 	P.dnls_sites = sites, P.dnls_radius = R;
@@ -1106,12 +1124,12 @@ extern "C" int nlc_plan_create(const nlc_model *model, nlc_plan **out) {
 		}
 		if (!P->rs.blocks) {
 			// longer than one block's registers hold, or faster so: windows of the chain, ping-ponging
-			// between the caller's buffer and a second one of the same size
+			// between the caller's buffer and a second one
 			P->rs = window_shape(*P, mdl, P->variant, force_win ? std::atoi(force_win) : 0);
 			if (!P->rs.blocks) return set_error(NLC_EUNSUPPORTED, "no launchable integrator shape for this chain_length");
 			P->win_len = uint32_t(P->rs.lanes) * P->rs.sites;
 			P->win_steps = std::max<uint32_t>(1, P->win_len / 140);   // discarded ends: 5% of a window each
-			if ((rc = P->dalloc(&P->d_win, size_t(model->copies) * n))) {
+			if ((rc = window_buffer(*P))) {
 				if (!block.blocks) return rc;
 				cudaGetLastError();
 				P->rs = block, P->win_len = 0;
@@ -1334,40 +1352,56 @@ int nlc::move_rounds(nlc_plan *P, void *state, uint64_t rounds, uint32_t round_s
 	return NLC_OK;
 }
 
-int nlc::move_segment(nlc_plan *P, void *state, uint32_t steps, uint32_t seg, cudaStream_t st) {
-	if (!P || !state) return set_error(NLC_EINVAL, "NULL argument");
-	if (!steps) return NLC_OK;
-	if (P->m.model == NLC_DNLS && P->dnls_stencil && P->win_len) {
-		// windows: launches of at most win_steps steps (open segments in between), each reading one
-		// buffer and writing the interiors of its windows to the other
-		const uint32_t n = P->m.chain_length;
-		double2 *in = static_cast<double2 *>(state), *out = P->d_win;
-		DnlsStencilArgs a = P->sa;
+// Windows: launches of at most win_steps steps (open segments in between), each reading one buffer and
+// writing the interiors of its windows to the other; `launch` takes the launch's arguments, its input and
+// its windows.  The chains that the second buffer holds at a time, the passes in order on the stream.
+template <class Args, class Launch>
+static int move_windows(nlc_plan *P, void *state, Args a, uint32_t reach, uint32_t steps, uint32_t seg, cudaStream_t st,
+                        const Launch &launch) {
+	const uint32_t n = P->m.chain_length;
+	for (uint32_t first = 0; first < P->m.copies; first += P->win_copies) {
+		double2 *const chains = static_cast<double2 *>(state) + size_t(first) * n;
+		double2 *in = chains, *out = P->d_win;
+		a.copies = std::min(P->win_copies, P->m.copies - first);
 		for (uint32_t done = 0; done < steps;) {
 			const uint32_t s = std::min(steps - done, P->win_steps);
 			a.steps = s;
 			a.seg = ((done || (seg & NLC_SEG_CONTINUE)) ? NLC_SEG_CONTINUE : 0u) |
 			        ((done + s < steps || (seg & NLC_SEG_OPEN)) ? NLC_SEG_OPEN : 0u);
 			a.win_len = P->win_len;
-			a.win_halo = 7 * uint32_t(P->dnls_radius) * s;
+			a.win_halo = reach * s;
 			a.win_inner = P->win_len - 2 * a.win_halo;
 			a.win_count = (n + a.win_inner - 1) / a.win_inner;
 			a.win_out = out;
-			const unsigned long long units = (unsigned long long) P->m.copies * a.win_count;
-			const int blocks = int(std::min<unsigned long long>(
-			    units, (P->m.flags & NLC_FLAG_SHARED_GPU) ? 0x7fffffffull : (unsigned long long) P->dnls_blocks));
-			int rc = cuda_status(launch_dnls_stencil(a, in, P->dnls_radius, blocks, st),
-			                     "DNLS windowed stencil launch");
+			// one block per window for a shared GPU, else (`launch`) a persistent grid of the resident blocks
+			const unsigned long long units = (unsigned long long) a.copies * a.win_count;
+			const unsigned long long most = (P->m.flags & NLC_FLAG_SHARED_GPU)
+			                                    ? 0x7fffffffull
+			                                    : (unsigned long long) P->per_sm * P->prop.multiProcessorCount;
+			int rc = launch(a, in, int(std::min(units, most)));
 			if (rc) return rc;
 			std::swap(in, out);
 			done += s;
 		}
-		if (in != state)
-			return cuda_status(cudaMemcpyAsync(state, in, size_t(P->m.copies) * n * sizeof(double2),
-			                                   cudaMemcpyDeviceToDevice, st),
-			                   "windowed state copy");
-		return NLC_OK;
+		if (in != chains) {
+			int rc = cuda_status(cudaMemcpyAsync(chains, in, size_t(a.copies) * n * sizeof(double2),
+			                                     cudaMemcpyDeviceToDevice, st),
+			                     "windowed state copy");
+			if (rc) return rc;
+		}
 	}
+	return NLC_OK;
+}
+
+int nlc::move_segment(nlc_plan *P, void *state, uint32_t steps, uint32_t seg, cudaStream_t st) {
+	if (!P || !state) return set_error(NLC_EINVAL, "NULL argument");
+	if (!steps) return NLC_OK;
+	if (P->m.model == NLC_DNLS && P->dnls_stencil && P->win_len)
+		return move_windows(P, state, P->sa, 7 * uint32_t(P->dnls_radius), steps, seg, st,
+		                    [&](const DnlsStencilArgs &a, double2 *in, int blocks) {
+			                    return cuda_status(launch_dnls_stencil(a, in, P->dnls_radius, blocks, st),
+			                                       "DNLS windowed stencil launch");
+		                    });
 	if (P->m.model == NLC_DNLS && P->dnls_stencil) {
 		DnlsStencilArgs a = P->sa;
 		a.steps = steps;
@@ -1384,39 +1418,13 @@ int nlc::move_segment(nlc_plan *P, void *state, uint32_t steps, uint32_t seg, cu
 		                   "DNLS move launch");
 	}
 	RealArgs a = P->ra;
-	if (P->win_len) {
-		// windowed tier: launches of at most win_steps steps (open segments in between), each reading
-		// one buffer and writing the interiors of its windows to the other
-		const uint32_t n = P->m.chain_length;
-		double2 *in = static_cast<double2 *>(state), *out = P->d_win;
-		RealShape sh = P->rs;
-		for (uint32_t done = 0; done < steps;) {
-			const uint32_t s = std::min(steps - done, P->win_steps);
-			a.steps = s;
-			a.seg = ((done || (seg & NLC_SEG_CONTINUE)) ? NLC_SEG_CONTINUE : 0u) |
-			        ((done + s < steps || (seg & NLC_SEG_OPEN)) ? NLC_SEG_OPEN : 0u);
-			a.win_len = P->win_len;
-			a.win_halo = 7 * s;
-			a.win_inner = P->win_len - 2 * a.win_halo;
-			a.win_count = (n + a.win_inner - 1) / a.win_inner;
-			a.win_out = out;
-			const unsigned long long units = (unsigned long long) P->m.copies * a.win_count;
-			// persistent grid of the resident blocks, or one block per window for a shared GPU
-			sh.blocks = int(std::min<unsigned long long>(
-			    units, (P->m.flags & NLC_FLAG_SHARED_GPU) ? 0x7fffffffull
-			                                              : (unsigned long long) P->per_sm * P->prop.multiProcessorCount));
-			int rc = cuda_status(launch_real_move(P->m.model, P->variant, sh, reinterpret_cast<double *>(in), a, st),
-			                     "windowed move launch");
-			if (rc) return rc;
-			std::swap(in, out);
-			done += s;
-		}
-		if (in != state)
-			return cuda_status(cudaMemcpyAsync(state, in, size_t(P->m.copies) * n * sizeof(double2),
-			                                   cudaMemcpyDeviceToDevice, st),
-			                   "windowed state copy");
-		return NLC_OK;
-	}
+	if (P->win_len)
+		return move_windows(P, state, a, 7, steps, seg, st, [&](const RealArgs &w, double2 *in, int blocks) {
+			RealShape sh = P->rs;
+			sh.blocks = blocks;
+			return cuda_status(launch_real_move(P->m.model, P->variant, sh, reinterpret_cast<double *>(in), w, st),
+			                   "windowed move launch");
+		});
 	a.steps = steps;
 	a.seg = seg;
 	return cuda_status(launch_real_move(P->m.model, P->variant, P->rs, static_cast<double *>(state), a, st), "move launch");
