@@ -78,7 +78,9 @@ enum {
 	                                    small enough (propagator taps beyond 13 sites below 2^-64, dt up
 	                                    to ~0.15) and chain_length >= 2R + 2 (16 at dt = 0.01), each
 	                                    linear sub-step is the same operator applied as its real-space
-	                                    stencil (nlc_dnls_stencil_coefficients) */
+	                                    stencil (nlc_dnls_stencil_coefficients), but for 32 and 48 sites
+	                                    at R = 13 (dt from ~0.1).  The form follows from dt and
+	                                    chain_length alone, never from copies */
 };
 
 /*

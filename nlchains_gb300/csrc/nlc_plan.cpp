@@ -810,11 +810,13 @@ static int setup_dnls_stencil(nlc_plan &P) {
 	const int need = dnls_stencil_coefficients(P.m.dt, kMaxStencilRadius, a.c0m1, &a.taps[0][0], a.phase);
 	const int R = need <= 7 ? 7 : need <= 11 ? 11 : need <= kMaxStencilRadius ? kMaxStencilRadius : 0;
 	if (!R || n < uint32_t(2 * R + 2)) return NLC_OK;
-	// Many 32- or 48-site chains at radius 13: their three cheap passes (radix 4 twice, then 2 or 3) take
-	// less than the 54-operation stencil (5 steps of 16384 chains of 32 sites: 1.68 against 2.08 ms, of
-	// 4096: 0.52 against 0.55, of 2048: 0.42 against 0.29; 48 sites, 2048 chains: 0.52 against 0.56; 64
-	// sites, 16384 chains: 3.56 against 3.33)
-	if (R == 13 && (n == 32 || n == 48) && uint64_t(P.m.copies) * n >= (3u << 15)) return NLC_OK;
+	// At radius 13, lengths below four radii (most sites are stored a second time, as ghost cells) whose
+	// transform is two radix-4 passes and one of 2 or 3, 32 and 48, keep it: 5 steps of 16384 chains of 32
+	// sites 1.64 ms against 2.08 with the stencil, of 2048 chains of 48 sites 0.52 against 0.56 (36 sites
+	// 2.53 against 2.91 ms for 16384 chains, 9.52 against 9.16 for 65536; 64 sites 11.7 against 12.9; others
+	// 1.1 to 2.5 times slower).  At any number of copies, so that a chain's bits follow from its model
+	// alone, though the stencil has the lower latency for few chains (0.12 ms against 0.43 for 96).
+	if (R == 13 && n < 4u * R && n % 16 == 0) return NLC_OK;
 	int lanes = 0, sites = 0;
 	// NLC_DNLS_SITES=<E> restricts the shapes to E sites per lane (used by the tests to cover every
 	// instantiation); NLC_FORCE_WINDOW=<G> integrates in windows of G lanes where a block would hold
