@@ -101,10 +101,10 @@ NLC_HD int clz32(uint32_t x) {
 // ((hi 2^32 + lo) 2^(k - 64))^2 as a double, truncated toward zero to 53 bits (relative error below
 // 2^-51): the square the mode energies need, without the sign, the rounding step or an FP64
 // multiply.  |V| is normalised to its 64 leading bits m (the bits below are dropped), m^2 is taken
-// to its high 64 bits (without the product of the low halves: 2^-61), and those to a 53-bit mantissa.
-// |V| < 2^95, in 32-bit words with one branch, never taken but for |V| < 2^32: with 64-bit shifts and a
-// branch for either half the conversion took most of the projection's epilogue, 67 us of a 1024 x 4096
-// sample's 485 (with it and the read-out's conversions 461).
+// to its high 64 bits, and those to a 53-bit mantissa.
+// |V| < 2^95 (the projection's sums: below 2^85), in 32-bit words with one branch, never taken but for
+// |V| < 2^32: with 64-bit shifts and a branch for either half the conversion took most of the
+// projection's epilogue, 67 us of a 1024 x 4096 sample's 485 (with it and the read-out's conversions 463).
 NLC_HD double fixed128_square_to_double(long long hi, long long lo, int k) {
 	// V as three words of two's complement, then |V|
 	const unsigned long long low = (unsigned long long) (uint32_t) (lo >> 32) + (uint32_t) hi;
@@ -120,8 +120,10 @@ NLC_HD double fixed128_square_to_double(long long hi, long long lo, int k) {
 	const int lz = clz32(w2);
 	e -= lz;
 	const uint32_t m1 = funnel_left(w1, w2, lz), m0 = funnel_left(w0, w1, lz);
-	// |V| ~ m 2^(e - 63); V^2 ~ sq 2^(2e - 62) with sq ~ (m^2) >> 64 in [2^62, 2^64)
-	const unsigned long long sq = (unsigned long long) m1 * m1 + (((unsigned long long) m1 * m0) >> 31);
+	// |V| ~ m 2^(e - 63); V^2 ~ sq 2^(2e - 62) with sq = (m^2) >> 64 in [2^62, 2^64)
+	// = m1^2 + floor((m1 m0 + floor(m0^2 / 2^33)) / 2^31)
+	const unsigned long long cross = (unsigned long long) m1 * m0 + (((unsigned long long) m0 * m0) >> 33);
+	const unsigned long long sq = (unsigned long long) m1 * m1 + (cross >> 31);
 	const int top = (int) (sq >> 63);
 	const unsigned long long mant = sq << (1 - top);   // leading one at bit 63
 	// value = mant 2^(top - 1) 2^(2e - 62) 2^(2k - 128): unbiased exponent 63 + top - 1 + 2e - 190 + 2k

@@ -125,3 +125,23 @@ def test_square_truncates_within_two_ulp(square):
             assert got == 0
             continue
         assert got <= exact and (exact - got) < exact * Fraction(1, 2 ** 51), (hi, lo, k)
+
+
+def test_square_is_the_truncated_product_of_the_leading_bits(square):
+    """Bit for bit: |V|'s 64 leading bits squared, the product's 64 leading bits kept, then 53 of those."""
+    rng = random.Random(13)
+    cases = [(2 ** 48, 2 ** 57 - 1, -7), (2 ** 62 - 1, 2 ** 32 - 1, 0), (-(2 ** 62) + 1, 0, 3), (0, 1, 0), (0, -(2 ** 31), 1)]
+    for _ in range(40000):
+        hi = rng.randrange(-2 ** 62, 2 ** 62) >> rng.randrange(0, 62)
+        lo = rng.randrange(-2 ** 62, 2 ** 62) >> rng.randrange(0, 62)
+        cases.append((hi, lo, rng.randrange(-60, 60)))
+    for hi, lo, k in cases:
+        v = abs(hi * 2 ** 32 + lo)
+        if v == 0:
+            continue
+        e = v.bit_length() - 1
+        m = v << (63 - e) if e <= 63 else v >> (e - 63)
+        sq = m * m >> 64
+        drop = sq.bit_length() - 53
+        want = math.ldexp(float(sq >> drop), drop + 2 * e - 62 + 2 * k - 128)
+        assert square(hi, lo, k) == want, (hi, lo, k)
