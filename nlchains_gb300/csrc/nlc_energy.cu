@@ -17,7 +17,9 @@
 
 namespace nlc {
 
-template <int MODEL>
+// QUARTIC (DNKG, dDNKG): beta is not zero, and the site's part is q^2 (beta q^2 / 2 + m); without it, (m q) q:
+// where q^2 overflows, a diverged chain's energy stays infinite (0 x infinity would be NaN).
+template <int MODEL, bool QUARTIC = true>
 __global__ void energies_kernel(const double2 *__restrict__ state, const EnergyArgs a, const FpOnes ones,
                                 double *__restrict__ out) {
 	const unsigned long long chain = (unsigned long long) blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32;
@@ -44,8 +46,9 @@ __global__ void energies_kernel(const double2 *__restrict__ state, const EnergyA
 				const double x = fmul(a2, d, k1);
 				v = fadd(v, fsub(expm1(x), x, k1), k1);
 			} else {
-				const double q2 = fmul(q, q, k1), ms = MODEL == NLC_DDNKG ? fadd(a.mp2_site[s], m, k1) : m;
-				h = dfma(d, d, dfma(q2, dfma(b2, q2, ms), h));
+				const double ms = MODEL == NLC_DDNKG ? fadd(a.mp2_site[s], m, k1) : m;
+				const double q2 = fmul(q, QUARTIC ? q : ms, k1);
+				h = dfma(d, d, dfma(q2, QUARTIC ? dfma(b2, q2, ms) : q, h));
 			}
 		}
 	}
@@ -62,8 +65,9 @@ cudaError_t launch_energies(const EnergyArgs &a, const double2 *state, double *o
 	const auto k = a.model == NLC_DNLS    ? energies_kernel<NLC_DNLS>
 	               : a.model == NLC_FPUT  ? energies_kernel<NLC_FPUT>
 	               : a.model == NLC_TODA  ? energies_kernel<NLC_TODA>
-	               : a.model == NLC_DDNKG ? energies_kernel<NLC_DDNKG>
-	                                      : energies_kernel<NLC_DNKG>;
+	               : a.model == NLC_DDNKG ? (a.beta != 0. ? energies_kernel<NLC_DDNKG> : energies_kernel<NLC_DDNKG, false>)
+	               : a.beta != 0.         ? energies_kernel<NLC_DNKG>
+	                                      : energies_kernel<NLC_DNKG, false>;
 	k<<<(unsigned) blocks, 256, 0, stream>>>(state, a, FpOnes{}, out);
 	return cudaGetLastError();
 }

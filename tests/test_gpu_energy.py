@@ -53,3 +53,29 @@ def test_energy_drift_bounded(gpu, name, params):
     job.close()
     ctx.close()
     assert np.abs(e1 / e0 - 1).max() < 1e-8
+
+
+@pytest.mark.parametrize("name,params", [
+    ("DNKG", dict(m=1.0, beta=0.0)), ("DNKG", dict(m=0.0, beta=0.0)), ("DNKG", dict(m=0.5, beta=1.0)),
+    ("dDNKG", dict(beta=0.0)), ("dDNKG", dict(beta=1.0)), ("FPUT", dict(alpha=0.0, beta=0.0)),
+    ("FPUT", dict(alpha=0.0, beta=1.0)), ("DNLS", dict(beta=1.0))])
+@pytest.mark.parametrize("uniform", [False, True])
+def test_energies_of_diverged_chains(gpu, name, params, uniform):
+    """Squares that overflow: the energy is infinite, or finite where the definition's terms are, never NaN."""
+    n, copies = 40, 3
+    masses = ic.masses_uniform(n, seed=n) if name == "dDNKG" else None
+    state = np.zeros((copies, n, 2))
+    state[1, :, 0] = 1e160 if uniform else np.where(np.arange(n) == 11, -1e160, 0.0)
+    state[2] = 0.4 * np.random.default_rng(1).standard_normal((n, 2))
+    ctx = gpu.Context(0)
+    job = ctx.job(gpu.Model(name, n, copies, 0.05, masses=masses, **params), 10)
+    job.upload(state)
+    e = job.energies()
+    job.close()
+    ctx.close()
+    with np.errstate(over="ignore"):
+        exp = O.energies(O.Model(name, n, copies, 0.05, masses=masses, **params), state)
+    assert not np.isnan(exp).any()
+    assert np.array_equal(np.isinf(e), np.isinf(exp)) and not np.isnan(e).any()
+    fin = np.isfinite(exp)
+    assert np.abs(e[fin] - exp[fin]).max() <= 1e-12 * np.abs(exp[fin]).max()
