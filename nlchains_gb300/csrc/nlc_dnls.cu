@@ -31,8 +31,12 @@ __device__ __forceinline__ double2 nonlinear_rotate(double2 v, double neg_coef, 
 // one unit from the self-resetting counter, so all its teams run the same control flow (a team
 // past the last chain repeats the last one and does not store).
 // 64 registers a thread: four 256-thread chains (or eight 128-thread team blocks) per SM; the block
-// variant also runs with 512 threads when the chain's buffers live in global memory
-template <bool BLOCK>
+// variant also runs with 512 threads when the chain's buffers live in global memory.
+// INT: the transforms' first additions on the integer pipes, for which the 64 registers are short (412
+// bytes of spills against 68): faster where many warps share a scheduler and hide that (5 steps, 1024
+// sites x 2048 chains 9.6 -> 8.6 ms, 64 x 16384 3.45 -> 3.0, 500 x 1024 3.8 -> 3.4), slower where few
+// do (512 x 64 545 us without, 627 with; 16 x 4096 294 and 337; 1009 x 512, padded, 5.4 and 5.8 ms).
+template <bool BLOCK, bool INT>
 __global__ void __launch_bounds__(BLOCK ? 512 : 128, BLOCK ? 2 : 8) dnls_move_kernel(double2 *__restrict__ psi, const DnlsArgs a) {
 	extern __shared__ double2 sm[];
 	__shared__ unsigned long long s_chain[32];
@@ -81,9 +85,9 @@ __global__ void __launch_bounds__(BLOCK ? 512 : 128, BLOCK ? 2 : 8) dnls_move_ke
 				};
 				const double2 *tab = a.conv_tables ? a.conv_tables + (size_t) k * len : a.lin_tables + (size_t) k * n;
 				auto propagate = [&](int j, double2 v) { return cmul(v, tab[j], k1); };
-				double2 *r = stockham_team<BLOCK, false>(a.fft, k1, x, y, t, T, rotate, propagate);
+				double2 *r = stockham_team<BLOCK, false, INT>(a.fft, k1, x, y, t, T, rotate, propagate);
 				double2 *o = r == x ? y : x;
-				x = stockham_team<BLOCK, true>(a.fft, k1, r, o, t, T);
+				x = stockham_team<BLOCK, true, INT>(a.fft, k1, r, o, t, T);
 				y = x == buf0 ? buf1 : buf0;
 			}
 		}
@@ -111,8 +115,9 @@ __global__ void __launch_bounds__(BLOCK ? 512 : 128, BLOCK ? 2 : 8) dnls_move_ke
 cudaError_t launch_dnls_move(const DnlsArgs &a, double2 *psi, int blocks, int threads, size_t smem,
                              int team_block, cudaStream_t stream) {
 	count_launch();
-	if (team_block) dnls_move_kernel<true><<<blocks, threads, smem, stream>>>(psi, a);
-	else dnls_move_kernel<false><<<blocks, threads, smem, stream>>>(psi, a);
+	const auto k = team_block ? (a.mixed ? dnls_move_kernel<true, true> : dnls_move_kernel<true, false>)
+	                          : (a.mixed ? dnls_move_kernel<false, true> : dnls_move_kernel<false, false>);
+	k<<<blocks, threads, smem, stream>>>(psi, a);
 	return cudaGetLastError();
 }
 
@@ -149,7 +154,8 @@ cudaError_t launch_dnls_linear(double2 *psi, uint64_t elements, uint32_t n, cons
 }  // namespace nlc
 
 namespace nlc {
-const void *dnls_kernel_ptr(int team_block) {
-	return team_block ? (const void *) dnls_move_kernel<true> : (const void *) dnls_move_kernel<false>;
+const void *dnls_kernel_ptr(int team_block, bool mixed) {
+	return team_block ? (mixed ? (const void *) dnls_move_kernel<true, true> : (const void *) dnls_move_kernel<true, false>)
+	                  : (mixed ? (const void *) dnls_move_kernel<false, true> : (const void *) dnls_move_kernel<false, false>);
 }
 }  // namespace nlc

@@ -141,9 +141,9 @@ struct FftPlanDev {
 	const double2 *tw;     // tw[e] = exp(-2 pi i e / len), device
 	const double2 *gw;     // FMA-form twiddle entries of the radix-2/3/4 passes (fma_twiddle_entry), device
 	int gw_off[kMaxRadices];  // offset of pass r's entries in gw, in double2 units
-	// 1: the first pass's additions on the FP64 pipe: where zeros pad the inputs (the chirp-z transform
-	// and the convolution form: sums the integer pipes do not take), where the passes run from global
-	// memory, and where a scheduler has one warp or none (its integer and FP64 work do not overlap)
+	// 1: the first pass's additions on the FP64 pipe: where zeros pad the inputs (the chirp-z transform:
+	// sums the integer pipes do not take), where the passes run from global memory, and where a scheduler
+	// has one warp or none (its integer and FP64 work do not overlap)
 	int fp64_first;
 	int bluestein;         // 1: chirp-z transform through a length-m cyclic convolution
 	const double2 *chirp;  // exp(-i pi j^2 / n), j < n
@@ -239,6 +239,7 @@ struct DnlsArgs {
 	const double2 *conv_tables;  // [7][len] when set: the linear sub-steps as length-len cyclic convolutions
 	unsigned long long *work_counter;
 	int team;                  // lanes per chain of the warp-team variant (power of two, 4 .. 32)
+	int mixed;                 // 1: the transforms' first additions on the integer pipes
 	uint32_t seg;              // NLC_SEG_*
 	const double2 *sctab;      // (cos, sin)(2 pi j / 1024), j < 1024 (device)
 	SinCosConsts sc;

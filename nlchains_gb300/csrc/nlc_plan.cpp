@@ -792,7 +792,7 @@ int set_smem_attr(const void *k, size_t smem, const cudaDeviceProp &prop) {
 namespace nlc {
 const void *lin_kernel_ptr(int model, int team_block);
 const void *lin32_kernel_ptr(int team_block);
-const void *dnls_kernel_ptr(int team_block);
+const void *dnls_kernel_ptr(int team_block, bool mixed);
 }  // namespace nlc
 
 // Steps per launch of a windowed DNLS stencil launch: the discarded ends (7 R sites per step each)
@@ -945,9 +945,10 @@ static int setup_dnls_fourier(nlc_plan *P, const std::vector<double> &tab) {
 	}
 	const bool global = len > smem_fft_len(*P);   // the chain's two buffers in global memory
 	if (global) P->dnls_threads = 512, P->dnls_smem = 0;
-	const void *k = dnls_kernel_ptr(P->dnls_team_block);
-	if ((rc = set_smem_attr(k, P->dnls_smem, P->prop))) return rc;
-	int per_sm = 0;
+	const void *k = dnls_kernel_ptr(P->dnls_team_block, false);
+	for (bool mixed : {false, true})
+		if ((rc = set_smem_attr(dnls_kernel_ptr(P->dnls_team_block, mixed), P->dnls_smem, P->prop))) return rc;
+	int per_sm = 0;   // (of either: both have 64 registers)
 	if ((rc = cuda_status(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, P->dnls_threads, P->dnls_smem),
 	                      "occupancy")))
 		return rc;
@@ -957,6 +958,12 @@ static int setup_dnls_fourier(nlc_plan *P, const std::vector<double> &tab) {
 	P->per_sm = per_sm;
 	P->block_warps = P->dnls_threads / 32;
 	P->dnls_blocks = int(std::min<unsigned long long>((model->copies + teams - 1) / teams, (unsigned long long) per_sm * sms));
+	// the integer pipes from three warps per scheduler on (4096 sites x 256 chains at 2: 7.0 ms with, 6.9
+	// without; below, nlc_dnls.cu), but not from global memory.  Padded lengths have zeros for inputs and all
+	// additions on the FP64 pipe (fp64_first); of the two instantiations warp teams run the one faster, blocks the
+	// other (98 sites x 2000 chains 2.45 and 2.67 ms, 1009 x 512 5.80 and 5.38).
+	d.mixed = d.fft.bluestein ? !P->dnls_team_block
+	                          : !global && (unsigned long long) P->dnls_blocks * P->block_warps >= 12ull * sms;
 	if ((model->flags & NLC_FLAG_SHARED_GPU) && !global)   // one block per unit of work: a warp's chains per unit
 		P->dnls_blocks = int(std::min<unsigned long long>(
 		    P->dnls_team_block ? model->copies : (model->copies + (32 / d.team) - 1) / (32 / d.team) / 4 + 1,
