@@ -251,26 +251,31 @@ __global__ void __launch_bounds__(BLOCK ? 512 : 128) ic_kernel(double2 *__restri
 	double2 *x = BLOCK && a.gscratch ? a.gscratch + (size_t) blockIdx.x * 2 * len : sm + (size_t) team * 2 * len;
 	double2 *y = x + len;
 	const FpOnes k1 = in_register(a.fft.k1, lane_zero(a.fft.k1));
-	// the teams of a block go from one chain to the next together (a team past the last chain idles), and
+	// The teams of a block go from one chain to the next together (a team past the last chain idles), and
 	// share the excited modes of all its chains: a few modes per chain would leave most of a warp's
 	// lanes idle in the sincospi and the divisions, and only the excited modes and their mirrors go
-	// through the divisions (N = 128 x 65536 with 10 modes: 1230 -> 480 us)
+	// through the divisions (N = 128 x 65536 with 10 modes: 1230 -> 480 us).  Modes enough for a team's lanes
+	// are its own, and where they and their mirrors are as many as all modes, every mode is gone through once
+	// (N = 128 x 8192, all modes: 190 us, 240 shared).
+	const bool own = BLOCK || c.nmodes >= 32, every = 2 * c.nmodes >= a.n;
 	for (unsigned long long base = (unsigned long long) blockIdx.x * teams; base < a.copies;
 	     base += (unsigned long long) gridDim.x * teams) {
 		const unsigned long long chain = base + team;
 		const bool active = chain < a.copies;
 		const int pairs = int(min((unsigned long long) teams, a.copies - base)) * int(c.nmodes);
+		const int p0 = own ? t : threadIdx.x, p1 = own ? (active ? int(c.nmodes) : 0) : pairs, dp = own ? T : int(blockDim.x);
 		double2 *dst = state + chain * (unsigned long long) n;
 		if (a.model == NLC_DDNKG) {
 			// the excited eigenmodes' amplitudes into the team's nmodes slots, then each site sums them
 			double2 *amp = sm + (size_t) team * c.nmodes;
-			for (int p = threadIdx.x; p < pairs; p += blockDim.x) {
-				const int q = p / int(c.nmodes), k = c.modes[p - q * int(c.nmodes)];
+			for (int p = p0; p < p1; p += dp) {
+				const int q = own ? team : p / int(c.nmodes), j = own ? p : p - q * int(c.nmodes), k = c.modes[j];
 				double s, co;
 				sincospi(2. * ic_uniform(c.key, c.first_copy + base + q, n, k), &s, &co);
-				sm[p] = make_double2(c.amp * co / a.omega[k], c.amp * s);
+				sm[(size_t) q * c.nmodes + j] = make_double2(c.amp * co / a.omega[k], c.amp * s);
 			}
-			__syncthreads();
+			if (own) team_sync<BLOCK>();
+			else __syncthreads();
 			for (int site = t; active && site < n; site += T) {
 				double p = 0., q = 0.;
 				for (int j = 0; j < int(c.nmodes); j++) {
@@ -279,14 +284,15 @@ __global__ void __launch_bounds__(BLOCK ? 512 : 128) ic_kernel(double2 *__restri
 				}
 				dst[site] = make_double2(p, q);
 			}
-			__syncthreads();
+			if (own) team_sync<BLOCK>();
+			else __syncthreads();
 			continue;
 		}
 		for (int k = t; k < n; k += T) x[k] = y[k] = make_double2(0., 0.);
 		__syncthreads();
 		double2 *const buf = BLOCK && a.gscratch ? x : sm;   // the first team's buffers
-		for (int p = threadIdx.x; p < pairs; p += blockDim.x) {
-			const int q = p / int(c.nmodes), k = c.modes[p - q * int(c.nmodes)];
+		for (int p = p0; p < p1; p += dp) {
+			const int q = own ? team : p / int(c.nmodes), k = c.modes[own ? p : p - q * int(c.nmodes)];
 			double s, co;
 			sincospi(2. * ic_uniform(c.key, c.first_copy + base + q, n, k), &s, &co);
 			buf[(size_t) q * 2 * len + k] = make_double2(c.amp * co, c.amp * s);
@@ -296,9 +302,13 @@ __global__ void __launch_bounds__(BLOCK ? 512 : 128) ic_kernel(double2 *__restri
 		if (a.model != NLC_DNLS) {
 			// Phi + i Pi from z at the excited modes and their mirrors (zero elsewhere):
 			// Phi_k = (z_k + conj z_{n-k}) / (2 omega_k), Pi_k = (z_k - conj z_{n-k}) / (2i)
-			for (int p = threadIdx.x; p < 2 * pairs; p += blockDim.x) {
-				const int q = (p >> 1) / int(c.nmodes), j = c.modes[(p >> 1) - q * int(c.nmodes)];
-				const int k = p & 1 ? (j ? n - j : 0) : j;
+			for (int p = every ? t : threadIdx.x, end = every ? (active ? n : 0) : 2 * pairs; p < end; p += every ? T : int(blockDim.x)) {
+				int q = team, k = p;
+				if (!every) {
+					q = (p >> 1) / int(c.nmodes);
+					const int j = c.modes[(p >> 1) - q * int(c.nmodes)];
+					k = p & 1 ? (j ? n - j : 0) : j;
+				}
 				const double2 *z = buf + (size_t) q * 2 * len;
 				const double2 zk = z[k], zc = make_double2(z[k ? n - k : 0].x, -z[k ? n - k : 0].y);
 				const double om = a.omega[k];
@@ -311,7 +321,7 @@ __global__ void __launch_bounds__(BLOCK ? 512 : 128) ic_kernel(double2 *__restri
 			w = y;
 		}
 		double2 *o = w == x ? y : x;
-		const double2 *r = fft_team<BLOCK, true>(a.fft, k1, w, o, t, T);
+		const double2 *r = fft_team<BLOCK, true, false>(a.fft, k1, w, o, t, T);
 		const double inv_n = in_register(1. / n, lane_zero(a.fft.k1));
 		for (int k = t; active && k < n; k += T) {
 			const double2 v = r[k];
@@ -321,10 +331,8 @@ __global__ void __launch_bounds__(BLOCK ? 512 : 128) ic_kernel(double2 *__restri
 	}
 }
 
-cudaError_t launch_initial_state(const DiagArgs &diag, const IcArgs &c, double2 *state, int blocks, int threads,
+cudaError_t launch_initial_state(const DiagArgs &a, const IcArgs &c, double2 *state, int blocks, int threads,
                                  size_t smem, int team_block, cudaStream_t stream) {
-	DiagArgs a = diag;
-	a.fft.fp64_first = 1;   // the spectrum is mostly zeros
 	// dDNKG: warp teams, shared memory for the excited modes' amplitudes; otherwise the transform's
 	// teams and buffers of the diagnostics
 	const bool block = a.model != NLC_DDNKG && team_block;

@@ -95,3 +95,43 @@ def test_server_seeded_request_equals_job(gpu):
     assert np.array_equal(fstate.reshape(copies, n, 2), job.download().reshape(copies, n, 2))
     job.close()
     ctx.close()
+
+
+@pytest.mark.parametrize("name,params,m", [("DNKG", dict(m=1.0, beta=1.0), 1.0), ("DNLS", dict(beta=1.0), None)])
+@pytest.mark.parametrize("n", [64, 100, 459])
+@pytest.mark.parametrize("count", [31, 32, "below half", "half", "all"])
+def test_many_modes(gpu, name, params, m, n, count):
+    """Modes enough for a team's lanes of its own (32), and as many, with their mirrors, as all modes (half);
+    warp teams with a partial last block, and a block per chain (459)."""
+    torch = pytest.importorskip("torch")
+    copies, seed, first, density = 33, 5, 2, 0.3
+    half = (n + 1) // 2
+    count = {"below half": half - 1, "half": half, "all": n}.get(count, count)
+    modes = np.arange(n - count, n) if count < n else np.arange(n)
+    plan = gpu.Plan(gpu.Model(name, n, copies, 0.05, **params))
+    dev = torch.zeros((copies, n, 2), dtype=torch.float64, device="cuda")
+    plan.initial_state(dev.data_ptr(), seed, density, modes, first_copy=first,
+                       stream=torch.cuda.current_stream().cuda_stream)
+    got = dev.cpu().numpy()
+    plan.close()
+    if name == "DNLS":
+        exp = ic.dnls_ensemble(n, copies, density, modes, seed=seed, first_copy=first).view(np.float64)
+    else:
+        exp = ic.real_ensemble(n, copies, density, modes, m=m, seed=seed, first_copy=first)
+    exp = np.asarray(exp).reshape(copies, n, 2)
+    assert np.abs(got - exp).max() <= 1e-12 * np.abs(exp).max()
+
+
+@pytest.mark.parametrize("nmodes", [31, 32, 64])
+def test_ddnkg_many_modes(gpu, nmodes):
+    torch = pytest.importorskip("torch")
+    n, copies, seed, density = 64, 33, 9, 0.5
+    masses = ic.masses_uniform(n, seed=3)
+    plan = gpu.Plan(gpu.Model("dDNKG", n, copies, 0.05, masses=masses, beta=1.0))
+    dev = torch.zeros((copies, n, 2), dtype=torch.float64, device="cuda")
+    plan.initial_state(dev.data_ptr(), seed, density, np.arange(nmodes), stream=torch.cuda.current_stream().cuda_stream)
+    got = dev.cpu().numpy()
+    plan.close()
+    mdl = O.Model("dDNKG", n, copies, 0.05, masses=masses, beta=1.0)
+    exp = O.linenergies(mdl, ic.ddnkg_ensemble(masses, copies, density, nmodes, seed=seed))
+    assert np.abs(O.linenergies(mdl, got) - exp).max() <= 1e-10 * np.abs(exp).max()
