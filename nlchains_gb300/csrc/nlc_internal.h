@@ -323,6 +323,24 @@ struct TcArgs {
 	unsigned long long wait_ns;  // limit of every mbarrier wait (wall clock)
 	int wait_test;             // tests only: thread 0 first waits on a barrier nothing arrives at
 };
+// Tiles beyond the last full wave: where they leave at least half of the SMs idle, each goes to
+// several blocks that share its read-out chunks (256 sites) of K (1024 x 256 samples 141 -> 82 us,
+// 1024 x 4096 512 -> 481, 700 x 2000 209 -> 177; tiles that fill more than half of the SMs gain nothing).
+struct TcSplit {
+	size_t whole, parts, rest;   // tiles taken whole, blocks per tile of the rest, those tiles
+};
+inline TcSplit tc_split(size_t tiles, size_t kp, size_t sms) {
+	const size_t rest = tiles % sms, chunks = (kp + 255) / 256;
+	const size_t parts = rest ? (chunks < sms / rest ? chunks : sms / rest) : 1;
+	return parts > 1 ? TcSplit{tiles - rest, parts, rest} : TcSplit{tiles, 1, 0};
+}
+// device bytes of the projection's buffers: the slices of X and E, the parked and the parts' sums
+inline size_t tc_projection_bytes(size_t n, size_t copies, size_t slices, size_t sms) {
+	const size_t mp = (2 * copies + 127) / 128 * 128, np = (n + 127) / 128 * 128, kp = (n + 15) / 16 * 16;
+	const TcSplit s = tc_split(mp / 128 * (np / 128), kp, sms);
+	const size_t tile = 128 * 128 * sizeof(long long), park = slices == 7 ? (s.whole + s.rest * s.parts) * tile : 0;
+	return slices * (mp + np) * kp * 2 + park + s.rest * s.parts * tile;
+}
 inline size_t tc_projection_tiles(const TcArgs &a) { return size_t(a.mp / 128) * (a.np / 128); }
 inline size_t tc_projection_blocks(const TcArgs &a) { return a.whole + (tc_projection_tiles(a) - a.whole) * a.parts; }
 cudaError_t launch_tc_projection(const TcArgs &a, const double2 *state, cudaStream_t stream);

@@ -616,22 +616,23 @@ int setup_tc_projection(nlc_plan &P, const double *d_omega, int slices) {
 	if ((rc = P.upload(&d_a, zeros.data(), zeros.size()))) return rc;
 	if ((rc = P.dalloc(&d_rexp, 2ull * P.m.copies))) return rc;
 	long long *d_park = nullptr;
-	// Tiles beyond the last full wave: where they leave at least half of the SMs idle, each goes to
-	// several blocks that share its read-out chunks (256 sites) of K (1024 x 256 samples 141 -> 82 us,
-	// 1024 x 4096 512 -> 481, 700 x 2000 209 -> 177; tiles that fill more than half of the SMs gain nothing).
-	const size_t sms = size_t(P.prop.multiProcessorCount), tiles = tc_projection_tiles(t), rest = tiles % sms;
-	t.parts = rest ? int(std::min<size_t>((t.kp + 255) / 256, sms / rest)) : 1;
-	t.whole = int(t.parts > 1 ? tiles - rest : tiles);
-	if (t.parts > 1 && P.dalloc(&t.part_sums, rest * t.parts * 128 * 128)) {
-		cudaGetLastError();
-		t.parts = 1, t.whole = int(tiles);   // no memory for the parts' sums
+	const size_t tiles = tc_projection_tiles(t);
+	TcSplit split = tc_split(tiles, size_t(t.kp), size_t(P.prop.multiProcessorCount));
+	for (;;) {   // whole tiles where there is no memory for the parts' sums
+		const size_t held = P.allocs.size();
+		t.whole = int(split.whole), t.parts = int(split.parts);
+		rc = t.parts > 1 ? P.dalloc(&t.part_sums, split.rest * split.parts * 128 * 128) : NLC_OK;
+		if (!rc && slices == 7) rc = P.dalloc(&d_park, tc_projection_blocks(t) * 128 * 128);
+		if (!rc) break;
+		if (t.parts == 1) return rc;
+		for (; P.allocs.size() > held; P.allocs.pop_back()) cudaFreeAsync(P.allocs.back(), cudaStreamLegacy);
+		split = TcSplit{tiles, 1, 0};
 	}
 	if (t.parts > 1) {
-		const std::vector<unsigned int> zero(2 * rest, 0);
+		const std::vector<unsigned int> zero(2 * split.rest, 0);
 		if ((rc = P.upload(&t.part_count, zero.data(), zero.size()))) return rc;
-		t.part_fail = reinterpret_cast<int *>(t.part_count + rest);
+		t.part_fail = reinterpret_cast<int *>(t.part_count + split.rest);
 	}
-	if (slices == 7 && (rc = P.dalloc(&d_park, tc_projection_blocks(t) * 128 * 128))) return rc;
 	const int zero = 0;
 	if ((rc = P.upload(&d_status, &zero, 1))) return rc;
 	t.a_slices = d_a, t.b_slices = d_b, t.row_exp = d_rexp, t.col_exp = d_fexp, t.omega = d_omega, t.status = d_status,

@@ -128,6 +128,7 @@ struct nlc_server {
 	std::condition_variable cv_prepare;
 	cudaStream_t free_stream = nullptr;   // final read-backs and frees only: never holds queued kernels
 	double quantum_us = 3000;
+	int sms = 1;   // of the device
 	std::vector<cudaStream_t> streams;
 	std::vector<int> slot_band;   // priority band of each stream slot, 0 = the highest stream priority
 	std::vector<cudaEvent_t> events;
@@ -573,6 +574,9 @@ extern "C" int nlc_server_create(const nlc_server_config *config, nlc_server **o
 	S->quantum_us = S->cfg.quantum_ms > 0 ? S->cfg.quantum_ms * 1e3 : S->cfg.quantum_ms < 0 ? 0. : 3000.;
 	int rc = cuda_status(cudaSetDevice(S->cfg.device), "cudaSetDevice");
 	if (rc) return rc;
+	if ((rc = cuda_status(cudaDeviceGetAttribute(&S->sms, cudaDevAttrMultiProcessorCount, S->cfg.device),
+	                      "cudaDeviceGetAttribute")))
+		return rc;
 	if (!S->cfg.hbm_budget_bytes) {
 		size_t fr = 0, tot = 0;
 		if ((rc = cuda_status(cudaMemGetInfo(&fr, &tot), "cudaMemGetInfo"))) return rc;
@@ -703,14 +707,10 @@ int submit(nlc_server *S, const nlc_model *model, uint32_t batching, uint64_t st
 	                (n > 4096 ? R->state_bytes : 0);   // windowed integrators: a second state buffer
 	if (n > 4096) R->need_bytes += R->state_bytes + size_t(2 * 1024) * 4 * n * sizeof(double2);   // windows / FFT scratch
 	if (model->model == NLC_DDNKG) {
-		// the tensor-core projection (the plan's rule): BF16 slices of the state and of the
-		// eigenvectors, and with 7 slices the first sweep's integer sums
+		// the tensor-core projection (the plan's rule)
 		const bool bf16x3 = model->flags & NLC_FLAG_BF16X3_PROJECTION;
-		if (bf16x3 || (model->flags & NLC_FLAG_TENSOR_PROJECTION) || (n >= 128 && !(model->flags & NLC_FLAG_FP64_PROJECTION))) {
-			const size_t mp = (2ull * model->copies + 127) / 128 * 128, np = (size_t(n) + 127) / 128 * 128,
-			             kp = (size_t(n) + 15) / 16 * 16, slices = bf16x3 ? 3 : 7;
-			R->need_bytes += slices * (mp + np) * kp * 2 + (bf16x3 ? 0 : mp * np * 8);
-		}
+		if (bf16x3 || (model->flags & NLC_FLAG_TENSOR_PROJECTION) || (n >= 128 && !(model->flags & NLC_FLAG_FP64_PROJECTION)))
+			R->need_bytes += tc_projection_bytes(n, model->copies, bf16x3 ? 3 : 7, size_t(S->sms));
 	}
 	std::lock_guard<std::mutex> lk(S->mu);
 	if (!S->fatal.empty()) return set_error(NLC_ECUDA, "server stopped after a CUDA error: " + S->fatal);
