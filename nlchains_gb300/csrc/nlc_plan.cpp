@@ -277,6 +277,9 @@ RealShape heuristic_shape(const nlc_plan &P, int model, int variant) {
 // line is "device<TAB>model<TAB>variant<TAB>n<TAB>bucket<TAB>lanes<TAB>sites<TAB>threads"; lines
 // that do not parse or name a shape this library cannot launch are ignored.  A ninth field, the
 // measured time of one step of an ensemble of the bucket, feeds the choice of rounds per launch.
+// The device's name carries the revision of the integrators and of the tuner's input (raised when either
+// changes what is fastest), so that shapes and times measured on others are ignored as another device's.
+constexpr const char *kTuneRevision = " rev 2";
 struct TuneKey {
 	std::string device;
 	int model, variant;
@@ -368,7 +371,7 @@ bool fill_tune_state(double *scratch, size_t doubles) {
 // Time every launchable (G, threads) shape on a small-amplitude ensemble for a few steps (best of
 // three launches after a warm-up one); keep the fastest.  Small ensembles take the heuristic shape.
 RealShape autotune_shape(nlc_plan &P, int model, int variant) {
-	const TuneKey key{P.prop.name, model, variant, P.m.chain_length, copies_bucket(P.m.copies)};
+	const TuneKey key{std::string(P.prop.name) + kTuneRevision, model, variant, P.m.chain_length, copies_bucket(P.m.copies)};
 	{
 		std::lock_guard<std::mutex> lk(g_tune_mutex);
 		tune_cache_load();

@@ -55,3 +55,19 @@ def test_cache_off_writes_no_file(gpu, tmp_path):
     r = plan_in_new_process(env)
     assert r["launches"] > 0
     assert not list(tmp_path.rglob("shapes.tsv"))
+
+
+def test_shapes_of_another_revision_are_not_taken(gpu, tmp_path):
+    """A line of a library with other integrators (the device's plain name) is ignored: the shape is timed
+    anew, and the file gains a line that the next process takes."""
+    torch = pytest.importorskip("torch")
+    cache = tmp_path / "shapes.tsv"
+    env = dict(os.environ, NLC_TUNE_CACHE=str(cache))
+    old = f"{torch.cuda.get_device_name(0)}\t0\t1\t128\t10\t32\t4\t64\t1000\n"
+    cache.write_text(old)
+    first = plan_in_new_process(env)
+    assert first["launches"] > 0, "the old line's shape was taken"
+    lines = cache.read_text().splitlines(keepends=True)
+    assert lines[0] == old and len(lines) == 2
+    second = plan_in_new_process(env)
+    assert second["launches"] == 0 and second["shape"] == first["shape"]
