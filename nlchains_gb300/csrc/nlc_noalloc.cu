@@ -194,6 +194,8 @@ extern "C" int nlc_linenergies_noalloc(int32_t model, uint32_t chain_length, uin
 	blocks = std::min<unsigned long long>(blocks, (512ull / threads) * S->sms);   // as many as the registers hold
 	blocks = std::min<unsigned long long>(blocks, rows_cap);
 	if (!blocks) return set_error(NLC_EINVAL, "nlc_linenergies_noalloc: scratch too small for this chain_length");
+	// as in a plan: with one warp per scheduler or two, the transforms' first additions stay on the FP64 pipe
+	g.fft.fp64_first = blocks * (threads / 32) < 8ull * S->sms;
 	g.fft.tw = tw;
 	g.fft.gw = gw;
 	if (model == NLC_DNLS) g.omega = ca;
