@@ -202,10 +202,12 @@ int nlc_dnls_stencil_coefficients(double dt, int32_t max_radius, int32_t *radius
 /* Launch shape chosen for the integrator: lanes per chain, sites per lane, threads per block, and
  * the tier: 1 = register-resident, a chain on G <= 32 lanes of a warp; 2 = register-resident, a
  * chain on one block of G > 32 lanes; 3 = DNLS, chains resident in shared memory (or, beyond it, in
- * per-block global scratch); 4 = windowed, chains longer than one block holds, integrated in
- * overlapping windows of G x E sites (lanes x sites per lane) between two state buffers; 5 = DNLS
- * in shared memory, G lanes taking E or E - 1 sites each, the linear sub-steps as real-space stencils; 6 = the
- * same for DNLS chains longer than one block holds, in overlapping windows of G x E sites. */
+ * per-block global scratch); 4 = windowed, chains longer than one block holds (8192 sites for DNKG,
+ * 6144 for FPUT and Toda, 4096 for dDNKG), or of 256 lanes or more where that is estimated faster,
+ * integrated in overlapping windows of G x E sites (lanes x sites per lane) between the state and a
+ * second buffer of at most 1 GiB; 5 = DNLS in shared memory, G lanes taking E or E - 1 sites each,
+ * the linear sub-steps as real-space stencils; 6 = the same for DNLS chains longer than one block
+ * holds (4096 sites), in overlapping windows of G x E sites. */
 int nlc_plan_shape(const nlc_plan *plan, int32_t *lanes_per_chain, int32_t *sites_per_lane,
                    int32_t *threads_per_block, int32_t *tier);
 

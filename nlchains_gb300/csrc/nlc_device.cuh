@@ -49,15 +49,6 @@ __device__ __forceinline__ ExpConsts in_register(const ExpConsts &c, int zero) {
 	r.c3 = in_register(c.c3, zero), r.c2 = in_register(c.c2, zero);
 	return r;
 }
-// the constants of sincos_table's small-angle series (the others, of its table branch, stay where
-// they are: most angles are small)
-__device__ __forceinline__ SinCosConsts in_register(const SinCosConsts &c, int zero) {
-	SinCosConsts r = c;
-	r.q3 = in_register(c.q3, zero), r.q5 = in_register(c.q5, zero), r.q7 = in_register(c.q7, zero);
-	r.q9 = in_register(c.q9, zero), r.w2 = in_register(c.w2, zero), r.w4 = in_register(c.w4, zero);
-	r.w6 = in_register(c.w6, zero), r.w8 = in_register(c.w8, zero);
-	return r;
-}
 
 __device__ __forceinline__ double fadd(double a, double b, const FpOnes &k) { return __fma_rn(a, k.one, b); }
 __device__ __forceinline__ double fsub(double a, double b, const FpOnes &k) { return __fma_rn(b, k.mone, a); }

@@ -53,7 +53,7 @@ struct IntAddend {
 };
 
 constexpr int kMaxSitesPerLane = 16;   // E: sites of a chain held in registers by one thread
-constexpr int kMaxLanesPerChain = 1024;
+constexpr int kMaxLanesPerChain = 512;   // the integrators' largest block
 
 // One ensemble inside a batched launch of the resident integrator (device table, see RealArgs).
 struct BatchJob {

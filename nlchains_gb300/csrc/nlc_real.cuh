@@ -3,7 +3,7 @@
 // Replaces the reference's three GPU tiers (move_chain_in_thread / move_chain_in_warp / move_split,
 // DNKG_FPUT_Toda.cu:82-259, dDNKG.cu:25-196) with one kernel family:
 //
-// * a chain of n sites is spread over G lanes (G a power of two, 1 .. 1024), each lane holding E or
+// * a chain of n sites is spread over G lanes (G a power of two, 1 .. 512), each lane holding E or
 //   E - 1 consecutive sites in registers (E a compile-time constant 1..16, so arrays index
 //   statically), the first n - G(E - 1) lanes holding E -- the reference's warp layout
 //   (DNKG_FPUT_Toda.cu:94-106) generalised to any group width;
@@ -185,7 +185,10 @@ __device__ __forceinline__ void sub_batch(double *out, const double *a, const do
 
 // Threads that a block may have, which caps the registers: at 512 (128 registers) four blocks of 128
 // threads share an SM, where the compiler's own choice of 130 to 138 leaves three (FPUT N = 459, 3001
-// chains, 50 steps: 4.82 -> 4.56 ms); more registers where 128 would spill.
+// chains, 50 steps: 4.82 -> 4.56 ms), for spills of up to 48 bytes (dDNKG's windows of 8: 132); more
+// registers where 128 would spill more, up to 824 bytes, of which 72 remain (Toda's windows of 16: 152).
+// A chain on one block is at most 512 lanes of 16 sites (DNKG), 12 (FPUT, Toda) or 8 (dDNKG); longer
+// ones run in windows.
 template <int MODEL, int E, bool WIN>
 constexpr int kMaxThreads = MODEL == NLC_DNKG    ? (WIN && E >= 12 ? 384 : 512)
                             : MODEL == NLC_DDNKG ? (E <= 8 ? 512 : E <= 11 ? 384 : 256)
@@ -193,7 +196,7 @@ constexpr int kMaxThreads = MODEL == NLC_DNKG    ? (WIN && E >= 12 ? 384 : 512)
 
 template <int MODEL, int E, int VAR, bool WIN>
 __global__ void __launch_bounds__(kMaxThreads<MODEL, E, WIN>) real_move_kernel_t(double2 *__restrict__ state, const RealArgs a) {
-	__shared__ double xbuf[4 * 32];
+	__shared__ double xbuf[4 * (kMaxLanesPerChain / 32)];
 	__shared__ double s_tab[MODEL == NLC_TODA ? kExpTable : 1];
 	__shared__ unsigned long long s_unit;
 	__shared__ int s_job;

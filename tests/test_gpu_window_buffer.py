@@ -37,3 +37,26 @@ def test_large_ensembles_need_no_second_state(gpu, name, n, copies, kw):
         assert torch.equal(part, base[:len(part)]), f"chains from {first} on"
     plan.close()
     small.close()
+
+
+@pytest.mark.parametrize("name,limit,kw", [("DNKG", 8192, dict(m=1.0, beta=1.0)), ("FPUT", 6144, dict(alpha=0.25, beta=0.5)),
+                                           ("Toda", 6144, dict(alpha=0.5))])
+def test_longest_chain_of_a_block(gpu, name, limit, kw):
+    """The longest chain that a block holds, and one site more, which runs in windows: bit for bit the oracle's."""
+    import oracle as O
+    copies, steps = 2, 3
+    for n, tier in ((limit, 2), (limit + 1, 4)):
+        state = 0.3 * np.random.default_rng(n).standard_normal((copies, n, 2))
+        model = gpu.Model(name, n, copies, 0.05, flags=gpu.FLAG_CANONICAL_SHAPE | gpu.FLAG_NO_TUNE, **kw)
+        plan = gpu.Plan(model)
+        assert plan.shape()["tier"] == tier
+        plan.close()
+        ctx = gpu.Context(0)
+        job = ctx.job(model, steps)
+        job.upload(state)
+        job.advance(steps)
+        out = job.download()
+        job.close()
+        ctx.close()
+        exp = O.advance(O.Model(name, n, copies, 0.05, **kw), state.copy(), steps, steps)
+        assert np.array_equal(np.asarray(out), np.asarray(exp).reshape(out.shape)), n
