@@ -55,13 +55,19 @@ __device__ __forceinline__ double2 rotate_phase(double2 v, double neg_coef, doub
 	return make_double2(dfma(v.x, c, -fmul(v.y, s, k)), dfma(v.x, s, fmul(v.y, c, k)));
 }
 
+// Rows that a warp computes on the FP64 pipe alone after one whose integer-pipe operations had to be
+// redone: where a chain is at rest, or its tails decay below the operands' range, every row would take both
+// forms (16384 sites x 64 chains with one site excited, 10 steps: 15.0 ms so, 8.9 with rows held).
+constexpr int kHoldRows = 12;
+
 // The same with the products of two varying factors on the integer pipes: 5 of the 17 operations of an
 // angle below 2^-4, 6 of the 21 of the table method, in warps whose angles are all of one kind (mixed
-// ones take sincos_table as it is); redone by rotate_phase where a lane's operands ask for it.  Every
-// lane of the warp calls it.
+// ones take sincos_table as it is); redone by rotate_phase where a lane's operands ask for it (`hold`, see
+// kHoldRows).  Every lane of the warp calls it.
 __device__ __forceinline__ double2 rotate_phase_mixed(double2 v, double neg_coef, double neg_phase,
                                                       const double2 *__restrict__ sctab, const SinCosConsts &C,
-                                                      const FpOnes &k) {
+                                                      const FpOnes &k, int &hold) {
+	if (hold) return rotate_phase(v, neg_coef, neg_phase, sctab, C, k);
 	IntFlags f;
 	const double th = dfma(neg_coef, dfma(v.x, v.x, int_mul(v.y, v.y, f)), neg_phase);
 	const int hi = __double2hiint(th) & 0x7fffffff;
@@ -85,7 +91,9 @@ __device__ __forceinline__ double2 rotate_phase_mixed(double2 v, double neg_coef
 		sincos_table(th, sctab, C, k, &s, &c);
 	}
 	const double2 r = make_double2(dfma(v.x, c, -int_mul(v.y, s, f)), dfma(v.x, s, int_mul(v.y, c, f)));
-	return __any_sync(0xffffffffu, f.bad()) ? rotate_phase(v, neg_coef, neg_phase, sctab, C, k) : r;
+	if (!__any_sync(0xffffffffu, f.bad())) return r;
+	hold = kHoldRows;
+	return rotate_phase(v, neg_coef, neg_phase, sctab, C, k);
 }
 
 }  // namespace
@@ -157,6 +165,7 @@ __global__ void __launch_bounds__(TEAM ? 128 : WIN ? 384 : 256, WIN ? 2 : (TEAM 
 	}
 	const int zero = lane_zero(a.k1);
 	const FpOnes k1 = in_register(a.k1, zero);
+	int hold = 0;   // rows yet to be computed on the FP64 pipe alone (kHoldRows; the same in all lanes)
 	auto rotate = [&](double2 v, int i) {
 		SinCosConsts sc;
 		sc.q3 = ser_sm[0], sc.q5 = ser_sm[1], sc.q7 = ser_sm[2], sc.q9 = ser_sm[3];
@@ -164,7 +173,7 @@ __global__ void __launch_bounds__(TEAM ? 128 : WIN ? 384 : 256, WIN ? 2 : (TEAM 
 		sc.shifter = ser_sm[8], sc.inv = ser_sm[9], sc.p1 = ser_sm[10], sc.p2 = ser_sm[11];
 		sc.s3 = ser_sm[12], sc.s5 = ser_sm[13], sc.c2 = ser_sm[14], sc.c4 = ser_sm[15];
 		const double2 c = rot_sm[i];
-		return rotate_phase_mixed(v, c.x, c.y, a.sctab, sc, k1);
+		return rotate_phase_mixed(v, c.x, c.y, a.sctab, sc, k1, hold);
 	};
 
 	auto sync = [] {
@@ -217,6 +226,7 @@ __global__ void __launch_bounds__(TEAM ? 128 : WIN ? 384 : 256, WIN ? 2 : (TEAM 
 			const int next = last ? 8 : k;   // the next rotation: the next sub-step's, or the launch's closing one
 #pragma unroll 1
 			for (int r = 0; r < rows; r++) {
+				if (hold) hold--;
 				const int s = r * G + lane;
 				const bool mine = !idle && s < len;
 				const double *w = in + (mine ? s : 0);
@@ -225,11 +235,15 @@ __global__ void __launch_bounds__(TEAM ? 128 : WIN ? 384 : 256, WIN ? 2 : (TEAM 
 				for (int c = 0; c < 2; c++) {
 					const double *own = w + c * pitch, *other = w + (1 - c) * pitch, *t = tp + c * (R + 1);
 					// the sums on the integer pipes; redone on the FP64 pipe where a lane's operands ask for it
-					IntFlags f;
-					auto int_sum = [&](double u, double v) { return int_add(u, v, f); };
 					auto fp64_sum = [&](double u, double v) { return fadd(u, v, k1); };
-					double v = stencil_component<R>(own, other, t, int_sum, fp64_sum);
-					if (__any_sync(0xffffffffu, f.bad())) v = stencil_component<R>(own, other, t, fp64_sum, fp64_sum);
+					double v = 0.;
+					if (!hold) {
+						IntFlags f;
+						auto int_sum = [&](double u, double v) { return int_add(u, v, f); };
+						v = stencil_component<R>(own, other, t, int_sum, fp64_sum);
+						if (__any_sync(0xffffffffu, f.bad())) hold = kHoldRows;
+					}
+					if (hold) v = stencil_component<R>(own, other, t, fp64_sum, fp64_sum);
 					if (c) y.y = v;
 					else y.x = v;
 				}
