@@ -22,7 +22,8 @@
 // The FP64 pipe is the bound, so the 2R sums and 5 of the rotation's products run on the integer pipes
 // (nlc_intfp.cuh, the same bits), 28 operations at R = 7 stay on the FP64 pipe, and every operand of
 // theirs is a vector register.  n = 1024, 8192 chains, 10 steps: 51.8 ms with all 47 on the FP64 pipe,
-// 32.9 with the sums moved (that pipe 99% busy), 28.4 with the products too (2.95 G site-steps/s).
+// 32.9 with the sums moved (that pipe 99% busy), 28.4 with the products too, 27.7 with rows held (kHoldRows;
+// 3.03 G site-steps/s).
 //
 // Layout: a chain in shared memory, real and imaginary rows, twice (a sub-step reads one buffer and
 // writes the other), the R elements at each end of a row repeating the ring's other end.  G lanes (up
