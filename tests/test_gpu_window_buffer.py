@@ -62,14 +62,17 @@ def test_large_ensembles_need_no_second_state(gpu, name, n, copies, kw):
 
 
 @pytest.mark.parametrize("name,limit,kw", [("DNKG", 8192, dict(m=1.0, beta=1.0)), ("FPUT", 6144, dict(alpha=0.25, beta=0.5)),
-                                           ("Toda", 6144, dict(alpha=0.5))])
+                                           ("Toda", 6144, dict(alpha=0.5)), ("dDNKG", 4096, dict(beta=1.0))])
 def test_longest_chain_of_a_block(gpu, name, limit, kw):
     """The longest chain that a block holds, and one site more, which runs in windows: bit for bit the oracle's."""
     import oracle as O
     copies, steps = 2, 3
+    flags = gpu.FLAG_CANONICAL_SHAPE | gpu.FLAG_NO_TUNE | (gpu.FLAG_FP64_PROJECTION if name == "dDNKG" else 0)
     for n, tier in ((limit, 2), (limit + 1, 4)):
         state = 0.3 * np.random.default_rng(n).standard_normal((copies, n, 2))
-        model = gpu.Model(name, n, copies, 0.05, flags=gpu.FLAG_CANONICAL_SHAPE | gpu.FLAG_NO_TUNE, **kw)
+        if name == "dDNKG":
+            kw = dict(kw, masses=np.random.default_rng(n + 1).uniform(1.0, 3.0, n))
+        model = gpu.Model(name, n, copies, 0.05, flags=flags, **kw)
         plan = gpu.Plan(model)
         assert plan.shape()["tier"] == tier
         plan.close()
